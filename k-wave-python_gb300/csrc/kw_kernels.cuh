@@ -141,6 +141,11 @@ struct AxisParams {
   int use_kspace;
   float pow1, pow2;
   float scale;    // 1 / N_total
+  // mixed-radix passes: what the rounding of scale left out, and per axis and
+  // frequency -scale x the gain of the axis's transform pair (null: none)
+  float scale_lo;
+  const float* eps[3];
+  float nab_kk;   // a typical |k|^2 of the grid (scaling of logarithms)
 };
 
 // Spectral operator for one column (ky, kz fixed) of the axis-0 pass.

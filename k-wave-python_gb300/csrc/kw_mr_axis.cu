@@ -1,0 +1,118 @@
+// Host side of the mixed-radix axis passes: pass kind, tile width, launch.
+#include "kw_mr_launch.cuh"
+
+#include <cmath>
+
+#define KW_MR_AXIS_DECL(name)                                                                                    \
+  cudaError_t kw_mr_axis_attr_##name(int smem);                                                                  \
+  cudaError_t kw_mr_axis_go_##name(dim3 grid, int threads, size_t smem, cudaStream_t st, const MrAxisParams* W,  \
+                                   const MrAxisParams* Ps, const int2* map);
+KW_MR_AXIS_DECL(fwd)
+KW_MR_AXIS_DECL(inv)
+KW_MR_AXIS_DECL(grad)
+KW_MR_AXIS_DECL(div)
+KW_MR_AXIS_DECL(nab)
+KW_MR_AXIS_DECL(gen)
+
+namespace {
+constexpr int kMrSmemMax = 160 * 1024;
+
+// Columns per block (a power of two) for `nbuf` column buffers of length L:
+// 16 (a row of a tile is then one 128-byte line) as long as three blocks of
+// plain passes fit an SM, fewer for long axes; halved down to 4 (one 32-byte
+// sector) while the grid would leave SMs without a block.
+int mr_tile_log2(const KwMrLen& L, int nbuf, long long ncoltot, int nitems, int nsm) {
+  int lg = 4;
+  while (lg > 0 && ((size_t)L.slots * sizeof(float2) << lg) * nbuf > 72 * 1024) --lg;
+  while (lg > 2 && ((ncoltot + (1 << lg) - 1) >> lg) * nitems < 2LL * nsm) --lg;
+  return lg;
+}
+}  // namespace
+
+bool kw_mr_axis_attr() {
+  return kw_mr_axis_attr_fwd(kMrSmemMax) == cudaSuccess && kw_mr_axis_attr_inv(kMrSmemMax) == cudaSuccess &&
+         kw_mr_axis_attr_grad(kMrSmemMax) == cudaSuccess && kw_mr_axis_attr_div(kMrSmemMax) == cudaSuccess &&
+         kw_mr_axis_attr_nab(kMrSmemMax) == cudaSuccess && kw_mr_axis_attr_gen(kMrSmemMax) == cudaSuccess;
+}
+
+// Parameters and launch shape of one pass along an axis: A in plain mode over
+// `nb` buffers, or its job list; nouter outer blocks of A.ncols columns; nsm
+// SMs to fill.
+cudaError_t kw_mr_axis_plan(const AxisParams& A, const KwMrLen& L, const float2* tw, int nouter, int nb, int nsm,
+                            KwMrAxisLaunch& X) {
+  MrAxisParams& W = X.W;
+  W.A = A;
+  W.L = L;
+  W.tw = tw;
+  W.dcols = kw_divu_make((uint32_t)A.ncols);
+  W.ncoltot = (uint32_t)A.ncols * (uint32_t)nouter;
+  W.gate = nullptr;
+  W.gate_end = 0;
+  int nitems = nb, nbuf = 1;
+  if (A.mode < 2) {
+    X.kind = A.mode == 0 ? MK_FWD : MK_INV;
+  } else {
+    const int D = A.ndim;
+    bool grad = A.njobs == D, div = A.njobs == D && (A.jobs[0].op == OP_DIV || A.jobs[0].op == OP_GRAD);
+    bool nab = A.njobs >= 1 && A.njobs <= 2;
+    int ni = 0;
+    for (int j = 0; j < A.njobs; ++j) {
+      const AxisJob& J = A.jobs[j];
+      grad &= J.in == B_P && J.out == j && J.op == OP_GRAD && J.axis == j;
+      div &= J.in == j && J.out == j && J.op == A.jobs[0].op && J.axis == j;
+      nab &= J.in == j && J.out == j && J.op == (j == 0 ? OP_NAB1 : OP_NAB2);
+      bool seen = false;
+      for (int i = 0; i < ni; ++i) seen |= W.inp[i] == J.in;
+      if (!seen) W.inp[ni++] = J.in;
+    }
+    // the inputs run in blocks of their own: no job may write another one's input
+    for (int j = 0; j < A.njobs; ++j)
+      for (int i = 0; i < ni; ++i)
+        if (A.jobs[j].out == W.inp[i] && A.jobs[j].in != W.inp[i]) return cudaErrorInvalidValue;
+    X.kind = grad ? MK_GRAD : div ? MK_DIV : nab ? MK_NAB : MK_GEN;
+    W.der = A.jobs[0].op;
+    nitems = grad ? 1 : div ? D : nab ? A.njobs : ni;
+    nbuf = (X.kind == MK_GRAD || X.kind == MK_GEN) ? 2 : 1;
+    if (X.kind == MK_NAB) {
+      // |k|^2 near 1 where most of the spectrum lies, so that its logarithm is
+      // small and keeps its low bits: a power of two near the mean |k|^2
+      const double kk = A.nab_kk > 0.f ? A.nab_kk : 1.0;
+      const int e = (int)std::lround(std::log2(kk));
+      W.nab_inv = (float)std::ldexp(1.0, -e);
+      W.nab_fac[0] = (float)std::exp2(0.5 * e * (double)A.pow1);
+      W.nab_fac[1] = (float)std::exp2(0.5 * e * (double)A.pow2);
+    }
+  }
+  W.lgT = mr_tile_log2(L, nbuf, W.ncoltot, nitems, nsm);
+  const int T = 1 << W.lgT;
+  int per = 0;
+  for (int l = 0; l < L.np; ++l) per = L.per[l] > per ? L.per[l] : per;
+  X.threads = (per * T + 31) / 32 * 32;
+  if (X.threads > 256) X.threads = 256;
+  X.smem = ((size_t)L.slots * sizeof(float2) << W.lgT) * nbuf;
+  if (X.smem > (size_t)kMrSmemMax) return cudaErrorInvalidValue;
+  W.gx = X.gx = (int)((W.ncoltot + T - 1) / T);
+  X.gy = nitems;
+  return cudaSuccess;
+}
+
+static cudaError_t axis_go(int kind, dim3 grid, int threads, size_t smem, cudaStream_t st, const MrAxisParams* W,
+                           const MrAxisParams* Ps, const int2* map) {
+  switch (kind) {
+    case MK_FWD: return kw_mr_axis_go_fwd(grid, threads, smem, st, W, Ps, map);
+    case MK_INV: return kw_mr_axis_go_inv(grid, threads, smem, st, W, Ps, map);
+    case MK_GRAD: return kw_mr_axis_go_grad(grid, threads, smem, st, W, Ps, map);
+    case MK_DIV: return kw_mr_axis_go_div(grid, threads, smem, st, W, Ps, map);
+    case MK_NAB: return kw_mr_axis_go_nab(grid, threads, smem, st, W, Ps, map);
+    default: return kw_mr_axis_go_gen(grid, threads, smem, st, W, Ps, map);
+  }
+}
+
+cudaError_t kw_mr_axis_launch(const KwMrAxisLaunch& X, cudaStream_t st) {
+  return axis_go(X.kind, dim3(X.gx, X.gy), X.threads, X.smem, st, &X.W, nullptr, nullptr);
+}
+
+cudaError_t kw_mr_axis_group_launch(int kind, int blocks, int threads, size_t smem, cudaStream_t st,
+                                    const MrAxisParams* Ps, const int2* map) {
+  return axis_go(kind, dim3(blocks), threads, smem, st, nullptr, Ps, map);
+}

@@ -14,6 +14,7 @@
 
 #include "../../include/kwave_gb300.h"
 #include "kw_kernels.cuh"
+#include "kw_mr_launch.cuh"
 
 #define KW_VERSION 100  // 0.1.0
 
@@ -98,6 +99,13 @@ struct kw_plan {
   bool axis_reg[3] = {false, false, false};
   int axis_regP[3] = {0, 0, 0}, axis_regE[3] = {0, 0, 0};
   bool rows_reg = false;
+  // mixed-radix register passes (kw_mr.cuh): axes and row stages whose length factors there
+  bool axis_mr[3] = {false, false, false}, rows_mr = false;
+  KwMrLen mr_axis[3], mr_row;
+  float2* d_mr_tw_axis[3] = {nullptr, nullptr, nullptr};
+  float2* d_mr_tw_row = nullptr;
+  uint32_t* d_mr_pos = nullptr;
+  float* d_eps[3] = {nullptr, nullptr, nullptr};  // AxisParams::eps
   // persistent TMA axis passes
   void* tma = nullptr;
   bool tma_axis[3] = {false, false, false};
@@ -122,13 +130,17 @@ struct kw_plan {
   // grouping: when set, the generic passes of a step are recorded here
   // instead of launched (kw_batch folds them into grouped launches)
   struct LaunchRec {
-    int kind;  // 0 generic rows, 1 generic axis pass, 2 another kernel
+    int kind;  // 0 generic rows, 1 generic axis pass, 2 another kernel, 3 mixed-radix rows, 4 mixed-radix axis pass
     RowsParams rp;
     AxisParams ap;
+    KwMrRowsLaunch mr;
+    KwMrAxisLaunch ma;
     int gx, gy, gz;
     size_t smem;
   };
   std::vector<LaunchRec>* rec_list = nullptr;
+  bool gated_src = false;  // recording steps that serve past the end of the sources (kw_batch)
+  int rec_nsm = 0;  // SMs a recorded mixed-radix launch should fill (the batch's share of them)
   // step graphs: one captured step per distinct launch sequence, replayed with
   // the step index read from d_tstep
   struct StepGraph {
@@ -251,6 +263,29 @@ static std::vector<float2> twiddles(int n, int count) {
     w[j] = make_float2((float)cos(a), (float)sin(a));
   }
   return w;
+}
+
+// Pass twiddles of a mixed-radix length: w_{r_l m_l}^{t k} at off[l] + k m[l] + t.
+static std::vector<float2> mr_twiddles(const KwMrLen& L) {
+  std::vector<float2> w;
+  for (int l = 0; l < L.np - 1; ++l)
+    for (int k = 0; k < L.r[l]; ++k)
+      for (int t = 0; t < L.m[l]; ++t) {
+        const double a = -2.0 * M_PI * (double)(t * k) / (double)(L.r[l] * L.m[l]);
+        w.push_back(make_float2((float)cos(a), (float)sin(a)));
+      }
+  return w;
+}
+
+// Padded slots of every frequency k (low half) and of M - k (high half; k = 0:
+// of M / 2, its own mirror, when that exists).
+static std::vector<uint32_t> mr_positions(const KwMrLen& L) {
+  const int M = L.n;
+  std::vector<uint32_t> pos(M), out(M);
+  for (int b = 0; b < L.q; ++b)
+    for (int j = 0; j < L.rl; ++j) pos[kw_mr_freq(L, b) + j * L.q] = (uint32_t)(b * L.mp + j);
+  for (int k = 0; k < M; ++k) out[k] = pos[k] | pos[k ? M - k : M % 2 ? 0 : M / 2] << 16;
+  return out;
 }
 
 extern "C" {
@@ -516,6 +551,83 @@ static void set_generic_geometry(kw_plan* p, int T_req, int R) {
   }
 }
 
+// Which lengths run on the mixed-radix passes (kw_mr.cuh): all that no
+// power-of-two kernel takes, and on 2-D grids and 3-D grids of up to 2^19
+// cells the power-of-two lengths too.  Those grids are bound by the latency of
+// each launch: 128^2 tissue 44 us a step against 60 on the TMA-fed kernels,
+// 512^2 70 against 85, 1024^2 120 against 169, 64^3 water 53 against 58; 128^3
+// tissue is the other way round (294 against 219).  KWAVE_GB300_MR=0: never,
+// =2: every length.
+static int setup_mr(kw_plan* p) {
+  if (p->generic_only) return KW_OK;
+  const char* env = getenv("KWAVE_GB300_MR");
+  const int mode = env ? atoi(env) : 1;
+  // 32-bit element offsets
+  if (mode == 0 || p->spec_elems >= (1LL << 31) || p->ntot >= (1LL << 31)) return KW_OK;
+  const bool every = mode >= 2 || p->D == 2 || p->ntot <= (1LL << 19);
+  const bool brief = p->ntot <= (1LL << 20);  // smallest radices (kw_mr_factor)
+  // one upload of all tables: twiddles, then positions, then gains, 16-byte aligned
+  std::vector<float> host;
+  auto push = [&](const void* src, size_t bytes) -> size_t {
+    const size_t at = (host.size() + 3) & ~(size_t)3;
+    host.resize(at + (bytes + 3) / 4);
+    memcpy(host.data() + at, src, bytes);
+    return at;
+  };
+  size_t at_tw[3] = {0, 0, 0}, at_eps[3] = {0, 0, 0}, at_row = 0, at_pos = 0;
+  bool any = false, has_eps[3] = {false, false, false};
+  auto push_eps = [&](int axis, const std::vector<double>& e) {  // -scale x eps, as the operator passes read it
+    std::vector<float> f(e.size());
+    for (size_t k = 0; k < e.size(); ++k) f[k] = (float)(-e[k] / (double)p->ntot);
+    at_eps[axis] = push(f.data(), f.size() * sizeof(float));
+    has_eps[axis] = true;
+  };
+  int E, Pt;
+  for (int a = 0; a < p->D - 1; ++a) {
+    if ((!every && kw_reg_shape(p->N[a], &E, &Pt)) || !kw_mr_factor(p->N[a], p->mr_axis[a], brief)) continue;
+    const std::vector<float2> w = mr_twiddles(p->mr_axis[a]);
+    at_tw[a] = push(w.data(), w.size() * sizeof(float2));
+    std::vector<double> e(p->N[a]);
+    kw_mr_gain(p->mr_axis[a], w.data(), e.data());
+    push_eps(a, e);
+    p->axis_mr[a] = any = true;
+  }
+  if (any && !kw_mr_axis_attr()) return fail(KW_ERR_CUDA, "mixed-radix kernel attributes: %s", cudaGetErrorString(cudaGetLastError()));
+  const bool reg_rows = p->even && kw_reg_shape(p->Mfft, &E, &Pt);
+  if ((every || !reg_rows) && p->Mfft <= KW_MR_MAXM && kw_mr_factor(p->Mfft, p->mr_row, brief)) {
+    const std::vector<float2> w = mr_twiddles(p->mr_row);
+    const std::vector<uint32_t> pos = mr_positions(p->mr_row);
+    at_row = push(w.data(), w.size() * sizeof(float2));
+    at_pos = push(pos.data(), pos.size() * sizeof(uint32_t));
+    // a real row's frequency k goes through the complex frequencies k and M - k
+    // alike, and an even row's odd part through its post twiddle
+    const int M = p->Mfft;
+    std::vector<double> c(M), e(p->H);
+    kw_mr_gain(p->mr_row, w.data(), c.data());
+    for (int k = 0; k < p->H; ++k) {
+      e[k] = 0.5 * (c[k % M] + c[(M - k % M) % M]);
+      if (!p->even) continue;
+      const double a = -2.0 * M_PI * (double)k / (double)p->L, wr = (float)cos(a), wi = (float)sin(a);
+      e[k] += 0.5 * (wr * wr + wi * wi - 1.0);
+    }
+    push_eps(p->D - 1, e);
+    p->rows_mr = true;
+  }
+  if (host.empty()) return KW_OK;
+  float* d = nullptr;
+  int rc = upload(p, &d, host.data(), host.size());
+  if (rc) return rc;
+  for (int a = 0; a < 3; ++a) {
+    if (a < p->D - 1 && p->axis_mr[a]) p->d_mr_tw_axis[a] = reinterpret_cast<float2*>(d + at_tw[a]);
+    if (has_eps[a]) p->d_eps[a] = d + at_eps[a];
+  }
+  if (p->rows_mr) {
+    p->d_mr_tw_row = reinterpret_cast<float2*>(d + at_row);
+    p->d_mr_pos = reinterpret_cast<uint32_t*>(d + at_pos);
+  }
+  return KW_OK;
+}
+
 int32_t kw_plan_finalize(kw_plan* p) {
   if (!p) return fail(KW_ERR_INVALID, "null plan");
   if (p->finalized) return fail(KW_ERR_STATE, "plan already finalized");
@@ -678,13 +790,14 @@ int32_t kw_plan_finalize(kw_plan* p) {
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&p->nsm, cudaDevAttrMultiProcessorCount, dev));
   }
+  if ((rc = setup_mr(p))) return rc;
   if (!p->generic_only) {
     const char* env = getenv("KWAVE_GB300_NO_TMA");
     const bool no_tma = env && env[0] == '1';
     // the TMA pass indexes a spectrum with 32-bit element offsets
     const bool fits32 = (long long)p->spec_elems < (1LL << 31);
     for (int a = 0; a < D - 1 && !no_tma && fits32; ++a) {
-      if (!kw_tma_supported(p->N[a])) continue;
+      if (p->axis_mr[a] || !kw_tma_supported(p->N[a])) continue;
       if (!p->tma) p->tma = kw_tma_plan_create();
       int E, Pt;
       kw_reg_shape(p->N[a], &E, &Pt);
@@ -866,6 +979,10 @@ static bool adjoint_rows_reg() {
   return on;
 }
 
+// Passes on the run-time-length shared-memory kernels (k_rows, k_axis).
+static bool generic_rows(const kw_plan* p) { return !p->rows_mr && !p->rows_reg; }
+static bool generic_axis(const kw_plan* p, int a) { return !p->axis_mr[a] && !p->tma_axis[a] && !p->axis_reg[a]; }
+
 static int launch_rows(kw_plan* p, int stage, int init, int t, int write_p, cudaStream_t st) {
   int crc = check_rows(p, stage, init);
   if (crc) return crc;
@@ -886,9 +1003,20 @@ static int launch_rows(kw_plan* p, int stage, int init, int t, int write_p, cuda
   for (int a = 0; a < 3; ++a) P.srcu_on[a] = p->srcu_on[a];
   P.rec_us = p->rec_us;
   P.init_r2c = p->init_r2c;
+  // (the wait test withholds a copy of the bulk-fed velocity stage)
+  const bool mr = p->rows_mr && !(p->wait_test && stage == ST_U && !init);
+  KwMrRowsLaunch X;
+  if (mr) {
+    X.W.Q = P;
+    X.W.L = p->mr_row;
+    X.W.tw = p->d_mr_tw_row;
+    X.W.pos = p->d_mr_pos;
+    kw_mr_rows_plan(stage, p->rec_list ? p->rec_nsm : p->nsm, X);
+  }
   if (p->rec_list) {
     kw_plan::LaunchRec r{};
-    r.kind = (p->rows_reg && (stage < ST_ADJ_A || adjoint_rows_reg())) ? 2 : 0;
+    r.kind = mr ? 3 : (p->rows_reg && (stage < ST_ADJ_A || adjoint_rows_reg())) ? 2 : 0;
+    if (mr) r.mr = X;
     r.rp = P;
     r.gx = (p->nrows + p->R - 1) / p->R;
     r.gy = r.gz = 1;
@@ -899,7 +1027,9 @@ static int launch_rows(kw_plan* p, int stage, int init, int t, int write_p, cuda
   size_t slot = 0;
   int rc = ev_begin(p, st, &slot);
   if (rc) return rc;
-  if (p->rows_reg && (stage < ST_ADJ_A || adjoint_rows_reg())) {
+  if (mr) {
+    CK(kw_mr_rows_launch(X, st));
+  } else if (p->rows_reg && (stage < ST_ADJ_A || adjoint_rows_reg())) {
     P.R = p->rows_R;
     P.ex_stride = p->rows_RS;
     // the power-law density stage keeps the divergence in shared memory (one
@@ -967,9 +1097,13 @@ static int launch_axis_plain(kw_plan* p, int axis, int inv, const int* bufs, int
   A.mode = inv ? 1 : 0;
   for (int i = 0; i < nb; ++i) A.plain[i] = bufs[i];
   const int nouter = (p->D == 3 && axis == 1) ? p->N[0] : 1;
+  KwMrAxisLaunch X;
+  if (p->axis_mr[axis])
+    CK(kw_mr_axis_plan(A, p->mr_axis[axis], p->d_mr_tw_axis[axis], nouter, nb, p->rec_list ? p->rec_nsm : p->nsm, X));
   if (p->rec_list) {
     kw_plan::LaunchRec r{};
-    r.kind = (p->tma_axis[axis] || p->axis_reg[axis]) ? 2 : 1;
+    r.kind = p->axis_mr[axis] ? 4 : (p->tma_axis[axis] || p->axis_reg[axis]) ? 2 : 1;
+    if (r.kind == 4) r.ma = X;
     r.ap = A;
     r.gx = (A.ncols + A.T - 1) / A.T;
     r.gy = nouter;
@@ -981,7 +1115,9 @@ static int launch_axis_plain(kw_plan* p, int axis, int inv, const int* bufs, int
   size_t slot = 0;
   int rc = ev_begin(p, st, &slot);
   if (rc) return rc;
-  if (p->tma_axis[axis]) {
+  if (p->axis_mr[axis]) {
+    CK(kw_mr_axis_launch(X, st));
+  } else if (p->tma_axis[axis]) {
     CK(kw_tma_launch(p->tma, axis, p->N[axis], nouter, nb, p->nsm, st, A, pdl_ok(p)));
   } else if (p->axis_reg[axis]) {
     const int E = p->axis_regE[axis], Pt = p->axis_regP[axis], T = 256 / Pt, n = p->N[axis];
@@ -1027,10 +1163,22 @@ static int launch_axis_ops(kw_plan* p, const AxisJob* jobs, int nj, cudaStream_t
   A.use_kspace = p->g.use_kspace;
   A.pow1 = (float)(p->g.alpha_power - 2.0);
   A.pow2 = (float)(p->g.alpha_power - 1.0);
-  A.scale = (float)(1.0 / (double)p->ntot);
+  const double scale = 1.0 / (double)p->ntot;
+  A.scale = (float)scale;
+  A.scale_lo = (float)(scale - (double)A.scale);
+  for (int a = 0; a < 3; ++a) A.eps[a] = p->d_eps[a];
+  {
+    double kk = 0.0;
+    for (int a = 0; a < p->D; ++a) kk += M_PI * M_PI / (3.0 * p->g.spacing[a] * p->g.spacing[a]);
+    A.nab_kk = (float)kk;
+  }
+  KwMrAxisLaunch X;
+  if (p->axis_mr[0])
+    CK(kw_mr_axis_plan(A, p->mr_axis[0], p->d_mr_tw_axis[0], 1, 0, p->rec_list ? p->rec_nsm : p->nsm, X));
   if (p->rec_list) {
     kw_plan::LaunchRec r{};
-    r.kind = (p->tma_axis[0] || p->axis_reg[0]) ? 2 : 1;
+    r.kind = p->axis_mr[0] ? 4 : (p->tma_axis[0] || p->axis_reg[0]) ? 2 : 1;
+    if (r.kind == 4) r.ma = X;
     r.ap = A;
     r.gx = (A.ncols + A.T - 1) / A.T;
     r.gy = r.gz = 1;
@@ -1041,7 +1189,9 @@ static int launch_axis_ops(kw_plan* p, const AxisJob* jobs, int nj, cudaStream_t
   size_t slot = 0;
   int rc = ev_begin(p, st, &slot);
   if (rc) return rc;
-  if (p->tma_axis[0]) {
+  if (p->axis_mr[0]) {
+    CK(kw_mr_axis_launch(X, st));
+  } else if (p->tma_axis[0]) {
     CK(kw_tma_launch(p->tma, 0, p->N[0], 1, 0, p->nsm, st, A, pdl_ok(p)));
   } else if (p->axis_reg[0]) {
     const int E = p->axis_regE[0], Pt = p->axis_regP[0], T = 256 / Pt, n = p->N[0];
@@ -1076,10 +1226,10 @@ static int enqueue_sources(kw_plan* p, int t, cudaStream_t st) {
 
 static void set_step_flags(kw_plan* p, int t) {
   const HostSrc& hp = p->hsrc[KW_S_P0];
-  p->srcp_on = hp.set && hp.mode == KW_SRC_ADDITIVE && t < hp.len;
+  p->srcp_on = hp.set && hp.mode == KW_SRC_ADDITIVE && (p->gated_src || t < hp.len);
   for (int a = 0; a < 3; ++a) {
     const HostSrc& h = p->hsrc[KW_S_U0 + a];
-    p->srcu_on[a] = a < p->D && h.set && h.mode == KW_SRC_ADDITIVE && t < h.len;
+    p->srcu_on[a] = a < p->D && h.set && h.mode == KW_SRC_ADDITIVE && (p->gated_src || t < h.len);
   }
   // bit a: u_a on the pressure grid is recorded (its spectrum buffer exists)
   p->rec_us = (t >= p->g.record_start) ? (p->record_mask >> KW_R_UX) & 0x7 : 0;
@@ -1318,8 +1468,8 @@ int32_t kw_plan_autotune(kw_plan* p, int32_t nsteps, void* stream, int32_t* T_ou
   if (!p->finalized) return fail(KW_ERR_STATE, "kw_plan_autotune before kw_plan_finalize");
   if (p->t != 0) return fail(KW_ERR_STATE, "kw_plan_autotune needs a plan at t = 0 (kw_plan_reset first)");
   bool gen_axis = false;
-  for (int a = 0; a < p->D - 1; ++a) gen_axis |= !p->tma_axis[a] && !p->axis_reg[a];
-  const bool gen_rows = !p->rows_reg;
+  for (int a = 0; a < p->D - 1; ++a) gen_axis |= generic_axis(p, a);
+  const bool gen_rows = generic_rows(p);
   const int k = std::min(std::max(2, (int)nsteps), p->g.Nt - 1);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if ((gen_axis || gen_rows) && k >= 2) {
@@ -1655,10 +1805,111 @@ static int batch_upload(kw_batch* b, const void* host, size_t bytes, void** out)
   return KW_OK;
 }
 
+// Plans whose passes all run on the mixed-radix kernels.
+static bool mr_all(const kw_plan* p) {
+  if (!p->rows_mr) return false;
+  for (int a = 0; a < p->D - 1; ++a)
+    if (!p->axis_mr[a]) return false;
+  return true;
+}
+
+// Grouped launches of mixed-radix plans.  While any member's k-space corrected
+// source is on, the steps of all members with such sources hold the source
+// passes; the kernels leave out a member whose source is over (gate, srcp_on).
+// So members whose bursts end at different steps keep one launch sequence.
+constexpr int kSrcKeyBits = 0xf;
+
+static int mr_source_bits(const kw_plan* p) {
+  int bits = 0;
+  if (p->hsrc[KW_S_P0].set && p->hsrc[KW_S_P0].mode == KW_SRC_ADDITIVE) bits |= 1;
+  for (int a = 0; a < p->D; ++a)
+    if (p->hsrc[KW_S_U0 + a].set && p->hsrc[KW_S_U0 + a].mode == KW_SRC_ADDITIVE) bits |= 2 << a;
+  return bits;
+}
+
+// Step keys of the batch m steps on (-1: the plan has ended); false when some
+// plan has a plain step there.
+static bool batch_keys(kw_batch* b, int m, const std::vector<int>& end, const std::vector<int>& eend, std::vector<int>& keys) {
+  bool on = false;
+  for (size_t i = 0; i < b->plans.size(); ++i) {
+    kw_plan* p = b->plans[i];
+    const int t = p->t + m;
+    keys[i] = -1;
+    if (t >= end[i]) continue;
+    if (step_eager(p, t, eend[i])) return false;
+    keys[i] = step_key(p, t);
+    on |= mr_all(p) && (keys[i] & kSrcKeyBits);
+  }
+  if (on)
+    for (size_t i = 0; i < b->plans.size(); ++i)
+      if (keys[i] >= 0 && mr_all(b->plans[i])) keys[i] |= mr_source_bits(b->plans[i]);
+  return true;
+}
+
+// Launch k of the members is one grouped launch where their sequences agree;
+// otherwise the longest remaining sequence goes first.  `chains` independent
+// sets of members run beside each other.
+struct MrGroup {
+  int kind;  // LaunchRec::kind 3 or 4
+  int stage, dim, akind;
+  int blocks = 0, threads = 0;
+  size_t smem = 0;
+  std::vector<MrRowsParams> rp;
+  std::vector<MrAxisParams> ap;
+  std::vector<int2> map;
+  MrRowsParams* d_rp = nullptr;
+  MrAxisParams* d_ap = nullptr;
+  int2* d_map = nullptr;
+};
+
+static void mr_groups(const std::vector<const std::vector<kw_plan::LaunchRec>*>& lists, std::vector<MrGroup>& out) {
+  std::vector<size_t> at(lists.size(), 0);
+  auto same = [](const kw_plan::LaunchRec& a, const kw_plan::LaunchRec& b) {
+    if (a.kind != b.kind) return false;
+    return a.kind == 3 ? a.mr.stage == b.mr.stage && a.mr.dim == b.mr.dim : a.ma.kind == b.ma.kind;
+  };
+  for (;;) {
+    size_t lead = 0, left = 0;
+    for (size_t i = 0; i < lists.size(); ++i)
+      if (lists[i]->size() - at[i] > left) {
+        left = lists[i]->size() - at[i];
+        lead = i;
+      }
+    if (!left) return;
+    const kw_plan::LaunchRec& h = (*lists[lead])[at[lead]];
+    MrGroup g;
+    g.kind = h.kind;
+    g.stage = h.mr.stage;
+    g.dim = h.mr.dim;
+    g.akind = h.ma.kind;
+    for (size_t i = 0; i < lists.size(); ++i) {
+      if (at[i] >= lists[i]->size() || !same((*lists[i])[at[i]], h)) continue;
+      const kw_plan::LaunchRec& r = (*lists[i])[at[i]++];
+      int nb;
+      if (h.kind == 3) {
+        nb = r.mr.blocks;
+        g.threads = std::max(g.threads, r.mr.threads);
+        g.smem = std::max(g.smem, r.mr.smem);
+        g.rp.push_back(r.mr.W);
+      } else {
+        nb = r.ma.gx * r.ma.gy;
+        g.threads = std::max(g.threads, r.ma.threads);
+        g.smem = std::max(g.smem, r.ma.smem);
+        g.ap.push_back(r.ma.W);
+      }
+      const int m = (int)(h.kind == 3 ? g.rp.size() : g.ap.size()) - 1;
+      for (int k = 0; k < nb; ++k) g.map.push_back(make_int2(m, k));
+    }
+    g.blocks = (int)g.map.size();
+    out.push_back(std::move(g));
+  }
+}
+
 // The graph of one batch step for the given per-plan keys (built on first use).
 // The steps of plans whose passes are all generic are recorded, and launch k
 // of every such plan runs in one grouped launch (rows and axis passes apart);
-// the other plans join as child graphs of their own step graphs.
+// so do the steps of plans on the mixed-radix kernels (mr_groups); the other
+// plans join as child graphs of their own step graphs.
 static int batch_graph(kw_batch* b, const std::vector<int>& keys, kw_batch::Graph** out) {
   for (auto& g : b->graphs)
     if (g.keys == keys) {
@@ -1679,12 +1930,28 @@ static int batch_graph(kw_batch* b, const std::vector<int>& keys, kw_batch::Grap
   for (size_t i = 0; i < n; ++i) {
     if (keys[i] < 0) continue;
     kw_plan* p = b->plans[i];
+    const bool mr = mr_all(p);
     p->rec_list = &lists[i];
+    p->rec_nsm = std::max(1, p->nsm / (int)n);
+    p->gated_src = mr && (keys[i] & kSrcKeyBits);
     p->capturing = true;
     rc = enqueue_step(p, p->t, false, nullptr);
     p->rec_list = nullptr;
+    p->gated_src = false;
     p->capturing = false;
     if (rc) return rc;
+    if (mr) {
+      int len = 0;
+      for (int sl : {KW_S_P0, KW_S_U0, KW_S_U1, KW_S_U2})
+        if (p->hsrc[sl].set && p->hsrc[sl].mode == KW_SRC_ADDITIVE) len = std::max(len, p->hsrc[sl].len);
+      for (auto& r : lists[i])
+        if (r.kind == 4 && r.ma.W.A.mode == 2 && r.ma.W.A.jobs[0].op == OP_SKAPPA) {
+          r.ma.W.gate = p->d_tstep;
+          r.ma.W.gate_end = len;
+        }
+      G.grouped[i] = 2;
+      continue;
+    }
     // only plans created for grouping (KW_DESC_GENERIC_FFT): on the same
     // kernels, separate branches measured faster than grouped launches
     bool ok = !lists[i].empty() && (p->g.flags & KW_DESC_GENERIC_FFT);
@@ -1703,7 +1970,7 @@ static int batch_graph(kw_batch* b, const std::vector<int>& keys, kw_batch::Grap
   size_t maxlen = 0;
   for (size_t i = 0; i < n; ++i)
     if (G.grouped[i]) {
-      maxlen = std::max(maxlen, lists[i].size());
+      if (G.grouped[i] == 1) maxlen = std::max(maxlen, lists[i].size());
       ticks.push_back(b->plans[i]->d_tstep);
     }
   // launch j of the members: one grouped launch per kind (rows, axis) and FFT
@@ -1717,7 +1984,7 @@ static int batch_graph(kw_batch* b, const std::vector<int>& keys, kw_batch::Grap
       long long total = 0;
       size_t smem = 0;
       for (size_t i = 0; i < n; ++i) {
-        if (!G.grouped[i] || lists[i].size() <= j || lists[i][j].kind != kind) continue;
+        if (G.grouped[i] != 1 || lists[i].size() <= j || lists[i][j].kind != kind) continue;
         const kw_plan::LaunchRec& r = lists[i][j];
         if ((kind == 0 ? r.rp.flen.n1 : r.ap.flen.n1) != 0 ? !sched : sched) continue;
         blk.push_back(make_int4((int)total, r.gx, r.gy, 0));
@@ -1743,6 +2010,25 @@ static int batch_graph(kw_batch* b, const std::vector<int>& keys, kw_batch::Grap
       q.blk = static_cast<int4*>(dblk);
       pend.push_back(q);
     }
+  std::vector<MrGroup> mrg;
+  {
+    std::vector<const std::vector<kw_plan::LaunchRec>*> ml;
+    for (size_t i = 0; i < n; ++i)
+      if (G.grouped[i] == 2) ml.push_back(&lists[i]);
+    mr_groups(ml, mrg);
+    for (MrGroup& g : mrg) {
+      void* d = nullptr;
+      if (g.kind == 3) {
+        if ((rc = batch_upload(b, g.rp.data(), g.rp.size() * sizeof(MrRowsParams), &d))) return rc;
+        g.d_rp = static_cast<MrRowsParams*>(d);
+      } else {
+        if ((rc = batch_upload(b, g.ap.data(), g.ap.size() * sizeof(MrAxisParams), &d))) return rc;
+        g.d_ap = static_cast<MrAxisParams*>(d);
+      }
+      if ((rc = batch_upload(b, g.map.data(), g.map.size() * sizeof(int2), &d))) return rc;
+      g.d_map = static_cast<int2*>(d);
+    }
+  }
   int** dticks = nullptr;
   if (!ticks.empty()) {
     void* d = nullptr;
@@ -1771,6 +2057,11 @@ static int batch_graph(kw_batch* b, const std::vector<int>& keys, kw_batch::Grap
                   : kw_axis_group_launch_0(q.total, q.smem, b->cap, aq, q.blk, q.m);
     if (elaunch == cudaSuccess) elaunch = e;
   }
+  for (const MrGroup& g : mrg) {
+    const cudaError_t e = g.kind == 3 ? kw_mr_rows_group_launch(g.stage, g.dim, g.blocks, g.threads, g.smem, b->cap, g.d_rp, g.d_map)
+                                      : kw_mr_axis_group_launch(g.akind, g.blocks, g.threads, g.smem, b->cap, g.d_ap, g.d_map);
+    if (elaunch == cudaSuccess) elaunch = e;
+  }
   if (dticks) k_step_tick_group<<<((int)ticks.size() + 127) / 128, 128, 0, b->cap>>>(dticks, (int)ticks.size());
   const cudaError_t el = elaunch != cudaSuccess ? elaunch : cudaGetLastError();
   cudaGraph_t graph = nullptr;
@@ -1779,7 +2070,7 @@ static int batch_graph(kw_batch* b, const std::vector<int>& keys, kw_batch::Grap
     if (graph) cudaGraphDestroy(graph);
     return fail(KW_ERR_CUDA, "batch capture: %s", cudaGetErrorString(el != cudaSuccess ? el : ec));
   }
-  G.nlaunch = (long long)pend.size() + (dticks ? 1 : 0);
+  G.nlaunch = (long long)(pend.size() + mrg.size()) + (dticks ? 1 : 0);
   for (size_t i = 0; i < n; ++i) {
     if (!sg[i]) continue;
     cudaGraphNode_t node;
@@ -1895,18 +2186,9 @@ static int batch_run(kw_batch* b, int nsteps, cudaStream_t st, bool plain_last) 
     eend[i] = plain_last ? end[i] : end[i] + 1;
     span = std::max(span, end[i] - p->t);
   }
+  std::vector<int> next(n);
   for (int s = 0; s < span; ++s) {
-    bool together = true;
-    for (size_t i = 0; i < n; ++i) {
-      kw_plan* p = b->plans[i];
-      keys[i] = -1;
-      if (p->t >= end[i]) continue;
-      if (step_eager(p, p->t, eend[i])) {
-        together = false;
-        continue;
-      }
-      keys[i] = step_key(p, p->t);
-    }
+    const bool together = batch_keys(b, 0, end, eend, keys);
     int rc;
     if (!together) {
       // a step with plain launches somewhere: each plan on its own, in order
@@ -1938,20 +2220,7 @@ static int batch_run(kw_batch* b, int nsteps, cudaStream_t st, bool plain_last) 
     // how many steps from here keep this key vector (all of them graph steps)
     int m = 1;
     if (b->loops) {
-      while (s + m < span) {
-        bool same = true;
-        for (size_t i = 0; i < n && same; ++i) {
-          kw_plan* p = b->plans[i];
-          const int t = p->t + m;
-          if (keys[i] < 0) {
-            same = t >= end[i];
-          } else {
-            same = t < end[i] && !step_eager(p, t, eend[i]) && step_key(p, t) == keys[i];
-          }
-        }
-        if (!same) break;
-        ++m;
-      }
+      while (s + m < span && batch_keys(b, m, end, eend, next) && next == keys) ++m;
       if (m >= 4 && (rc = batch_loop_graph(b, g))) return rc;
     }
     for (size_t i = 0; i < n; ++i)
@@ -2020,8 +2289,8 @@ int32_t kw_batch_autotune(kw_batch* b, int32_t nsteps, void* stream, int32_t* T_
     if (p->t != 0) return fail(KW_ERR_STATE, "kw_batch_autotune needs every plan at t = 0");
   bool any = false;
   for (kw_plan* p : b->plans) {
-    bool g = !p->rows_reg;
-    for (int a = 0; a < p->D - 1; ++a) g |= !p->tma_axis[a] && !p->axis_reg[a];
+    bool g = generic_rows(p);
+    for (int a = 0; a < p->D - 1; ++a) g |= generic_axis(p, a);
     any |= g;
   }
   int bestT = 0, bestN = 1, bestD = 1;
