@@ -3,19 +3,29 @@
 // with this file's kernels only.  The reference has no counterpart; its input
 // is the image of kwave/reconstruction/time_reversal.py:129-150.
 //
-// Tensor-core core (k_umma): one CTA of 128 threads computes a 128 x NT tile
+// Tensor-core core (k_umma): one CTA of nine warps computes a 128 x NT tile
 // D[m][n] = sum_k A(m, k) B(n, k) on the 5th-generation tensor cores:
-//   * the 128 threads gather 64-wide K chunks of A and B (bf16) into a
-//     two-stage shared-memory ring, in the canonical K-major layout without
-//     swizzle (core matrices of 8 rows x 16 bytes, 128 contiguous bytes each;
-//     LBO = 128 bytes between core matrices along K, SBO = 1024 bytes between
-//     8-row groups);
-//   * one thread issues tcgen05.mma (kind::f16, bf16 x bf16 -> f32, M = 128,
-//     N = NT, K = 16 per instruction) into an accumulator in tensor memory
-//     (TMEM, allocated by warp 0) and tcgen05.commit's each stage to an
-//     mbarrier, which the gatherers wait on before refilling that stage;
-//   * the epilogue reads the accumulator with tcgen05.ld (warp w owns TMEM
-//     lanes 32w..32w+31, one D row per thread).
+//   * eight warps gather 64-wide K chunks of A and B (bf16) with 16-byte
+//     cp.async copies into a shared-memory ring of two to six stages, in the
+//     128-byte swizzled layouts (rows of 64 values, their 16-byte pieces
+//     permuted by the row number mod 8): neighbouring lanes then copy
+//     neighbouring pieces of one row, from one line of global memory to
+//     distinct banks (without swizzle they took 22 shared-memory cycles a
+//     warp's copy instead of 4).  Each warp runs ahead
+//     by itself: the copies arrive on the stage's full barrier as they land, and
+//     a warp waits only for the tensor cores to have read the stage it refills;
+//   * one lane of the ninth warp waits for full, issues tcgen05.mma (kind::f16,
+//     bf16 x bf16 -> f32, M = 128, N = NT, K = 16 per instruction) into an
+//     accumulator in tensor memory (TMEM, allocated by warp 0) and
+//     tcgen05.commit's each stage to its empty barrier;
+//   * the epilogue reads the accumulator with tcgen05.ld (warps w and w + 4 own
+//     TMEM lanes 32w..32w+31, one D row per thread, and take 16-column groups
+//     in turn).
+// A gather is bound by the latency of its loads and by instruction issue, not
+// by the tensor cores.  Gathering a stage with all threads, waiting for it and
+// issuing its MMAs in turn left one chunk in flight: the 384 -> 128 channel
+// layer at 16 x 64^2 took 445 us for its weight gradient and 445 us for its
+// data gradient, now 113 and 156; 256 -> 256 at 4 x 32^2 forward 81, now 31.
 // Every mbarrier wait is bounded (2 s of global time); a timeout sets the
 // device error word, skips the epilogue and still frees the TMEM.
 //
@@ -35,13 +45,11 @@
 //          convolution is the same gather with the flipped, transposed
 //          weights and the output gradient as input.
 //   WGRAD  weight gradient, k = pixel (split over CTAs, partial tiles added
-//          with red.add): by default m = (tap, input channel), n = output
-//          channel on MN-major tiles -- both operands are contiguous along m
-//          and n in the NHWC tensors, so their 16-byte groups are copied as
-//          they are (instruction descriptor bits 15/16; LBO = 128 bytes between
-//          K core matrices, SBO = 1024 bytes between 8-element groups); the
-//          K-major form (m = output channel) transposes 8 x 8 blocks in
-//          registers instead.
+//          with red.add): m = (tap, input channel), n = output channel on
+//          MN-major tiles -- both operands are contiguous along m and n in the
+//          NHWC tensors, so their 16-byte groups are copied as they are
+//          (instruction descriptor bits 15/16; SBO between 8-k groups, LBO
+//          between 64-wide blocks).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -52,6 +60,7 @@
 #include <cstring>
 
 #include "../../include/kwave_gb300.h"
+#include "kw_fft.cuh"
 #include "kw_tma.cuh"
 
 int kw_internal_fail(int code, const char* msg);
@@ -63,25 +72,33 @@ using kwtma::mbar_init;
 using kwtma::mbar_wait;
 using kwtma::smem_u32;
 
-constexpr int kThreads = 128;
+constexpr int kThreads = 256;         // gather threads of k_umma (one more warp issues the MMAs)
 constexpr int kBM = 128;            // tile rows (TMEM lanes)
 constexpr int kBK = 64;             // K chunk per stage (bf16: 128 bytes per row)
 constexpr int kMaxNT = 256;         // tile columns (TMEM columns)
-constexpr uint32_t kSBO = 1024;     // 8-row group stride in a stage tile
-constexpr uint32_t kLBO = 128;      // K-adjacent core matrix stride
+constexpr int kMaxStages = 6;       // deepest shared-memory ring
 constexpr int kATile = kBM * kBK * 2;         // 16 KB
 constexpr uint64_t kWaitNs = 2000000000ull;
 constexpr int kErrUmmaTimeout = 0x55;
 
 // tcgen05 shared-memory matrix descriptor: K-major, no swizzle; lbo = bytes
 // between core matrices adjacent along K, sbo = bytes between 8-row groups.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo = kLBO, uint32_t sbo = kSBO) {
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
   uint64_t d = 0;
   d |= (uint64_t)((addr >> 4) & 0x3FFFu);
   d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
   d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
   d |= (uint64_t)1 << 46;  // descriptor version of the 5th-generation tensor cores
   return d;                // base offset 0, swizzle mode 0 (none)
+}
+
+// The same for the 128-byte swizzled layouts (tiles 1024-byte aligned).
+// K-major: rows of 64 k, 8-row groups 1024 bytes apart (LBO unused).
+__device__ __forceinline__ uint64_t smem_desc_k128(uint32_t addr) { return smem_desc(addr, 16, 1024) | (uint64_t)2 << 61; }
+// MN-major: rows of 64 m or n, 8-k groups 1024 bytes apart (SBO), 64-wide
+// blocks `block` bytes apart (LBO).
+__device__ __forceinline__ uint64_t smem_desc_mn128(uint32_t addr, uint32_t block) {
+  return smem_desc(addr, block, 1024) | (uint64_t)2 << 61;
 }
 
 // Halo-tile convolution (mode 3): a tile is 128 consecutive pixels of one
@@ -154,31 +171,28 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// Byte offset of the 16-byte chunk (row r, 8-wide K group kc) in a stage tile.
-__device__ __forceinline__ uint32_t chunk_off(int r, int kc) {
-  return (uint32_t)((r >> 3) * kSBO + kc * kLBO + (r & 7) * 16);
+// Byte offset of 16-byte piece q (0..7) of row r in a swizzled stage tile: rows
+// of 64 values (K-major: row = m or n, piece = 8 k; MN-major: row = k, piece =
+// 8 m or n of one 64-wide block, blocks kBlock bytes apart).
+constexpr uint32_t kBlock = kBK * 128;
+__device__ __forceinline__ uint32_t piece_off(int r, int q) { return (uint32_t)(r * 128 + ((q ^ (r & 7)) << 4)); }
+
+// 16-byte asynchronous copy to shared memory; `in` false: zeros (src is not read).
+__device__ __forceinline__ void cp16(unsigned char* dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
 }
+// The same through L1: the convolution input, which neighbouring taps read again.
+__device__ __forceinline__ void cp16_l1(unsigned char* dst, const void* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+// Arrive on `bar` once all of this thread's copies so far have landed (the
+// barrier counts the arrival as one of its expected ones).
+__device__ __forceinline__ void cp_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 __device__ __forceinline__ uint4 ldg16(const void* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
-
-// Word w (0..3) of a uint4, w known at compile time after unrolling.
-__device__ __forceinline__ uint32_t word_of(const uint4& v, int w) {
-  return w == 0 ? v.x : w == 1 ? v.y : w == 2 ? v.z : v.w;
-}
-
-// 8 x 8 bf16 transpose: in[j] holds 8 values of row j; out[i] gets element i
-// of every row.  Word q of out[i] pairs element i of rows 2q and 2q + 1,
-// picked with byte permutes (low halves for even i, high halves for odd i).
-__device__ __forceinline__ void transpose8(const uint4 (&in)[8], uint4 (&out)[8]) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint32_t sel = (i & 1) ? 0x7632u : 0x5410u;
-    uint32_t w[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) w[q] = __byte_perm(word_of(in[2 * q], i >> 1), word_of(in[2 * q + 1], i >> 1), sel);
-    out[i] = make_uint4(w[0], w[1], w[2], w[3]);
-  }
-}
 
 }  // namespace
 
@@ -186,7 +200,7 @@ __device__ __forceinline__ void transpose8(const uint4 (&in)[8], uint4 (&out)[8]
 // gather policies
 // ---------------------------------------------------------------------------
 struct UmmaArgs {
-  int mode;  // 0 GEMM, 1 CONV, 2 WGRAD, 3 CONV on halo tiles, 4 GEMM of MN-major operands, 5 WGRAD MN-major
+  int mode;  // 0 GEMM, 1 CONV, 3 CONV on halo tiles, 4 GEMM of MN-major operands, 5 WGRAD (MN-major)
   int M, N, K;
   int NT;    // tile columns (multiple of 16, <= 256)
   // GEMM
@@ -206,234 +220,238 @@ struct UmmaArgs {
   const __nv_bfloat16* dZ;   // WGRAD: output gradient [pixels][M]
   float* dW;                 // WGRAD: [M][N] f32, accumulated
   int ksplit;                // WGRAD: pixels per CTA; CONV split over K: K values per CTA (multiple of 64, 0: no split)
+  int stages;                // depth of the shared-memory ring
+  KwDivU dhw, dw;            // division by H W and W
 };
 
-// 16-byte chunk of the convolution input at pixel (b, y, x) of the output
-// grid shifted by tap, channels ci..ci+7 (zero outside the image); bimg is the
-// index of the image's first pixel, b * H * W.
-__device__ __forceinline__ uint4 conv_chunk_at(const UmmaArgs& a, int bimg, int y, int x, int tap, int ci) {
-  y += tap / 3 - 1;
-  x += tap % 3 - 1;
-  if (tap >= 9 || y < 0 || y >= a.H || x < 0 || x >= a.W) return make_uint4(0, 0, 0, 0);
-  if (ci < a.C1) return ldg16(a.X1 + ((long long)bimg + y * a.W + x) * a.C1 + ci);
-  const int w2 = a.W >> 1;
-  return ldg16(a.X2 + ((long long)(bimg >> 2) + (y >> 1) * w2 + (x >> 1)) * a.C2 + (ci - a.C1));
+// Bits of the nine taps (3 (dy + 1) + dx + 1) that stay inside the image at pixel (y, x).
+__device__ __forceinline__ uint32_t tap_mask(const UmmaArgs& a, int y, int x) {
+  uint32_t m = 0x1FFu;
+  if (y == 0) m &= ~0x007u;
+  if (y == a.H - 1) m &= ~0x1C0u;
+  if (x == 0) m &= ~0x049u;
+  if (x == a.W - 1) m &= ~0x124u;
+  return m;
 }
 
-// Per-thread state of the CONV operand gathers.  Thread tid fills the 8-wide
-// K group kc = (tid >> 3) & 7 of the tile rows r_i = (2 i + (tid >> 6)) * 8 +
-// (tid & 7), i < 8, in every chunk: their output pixels are decomposed once
-// per tile, and the group's (tap, channel) advances by 64 per chunk without
-// divisions.
+// 16-byte chunk of the convolution input at pixel (y, x) of image b of the
+// output grid shifted by tap, channels ci..ci+7 (the place is inside the image).
+__device__ __forceinline__ const __nv_bfloat16* conv_src(const UmmaArgs& a, int b, int y, int x, int tap, int ci) {
+  const int dy = tap / 3 - 1;
+  y += dy;
+  x += tap - 3 * dy - 4;
+  if (ci < a.C1) return a.X1 + ((long long)(b * a.H + y) * a.W + x) * a.C1 + ci;
+  return a.X2 + ((long long)(b * (a.H >> 1) + (y >> 1)) * (a.W >> 1) + (x >> 1)) * a.C2 + (ci - a.C1);
+}
+
+// Per-thread state of the operand gathers, worked out once per tile so that a
+// chunk takes a few instructions per copy.
+//   CONV: thread tid fills the 8-wide K group tid & 7 of the tile rows
+//   (tid >> 3) + 32 i, i < 4, in every chunk: their output pixels are fixed, and
+//   the group's (tap, channel) advances by 64 per chunk without divisions.
+//   WGRAD on MN-major tiles: thread tid fills the 8-wide (tap, channel) group
+//   m0 / 8 + (tid & 15), whose shift and channel are fixed, of the pixels
+//   (tid >> 4) + 16 i, i < 4, of every chunk.
 struct ConvRows {
-  int bimg[8];  // b * H * W of the row's pixel, -1 beyond the batch
-  int yx[8];    // y << 16 | x
-  int tap, ci;
-  __device__ __forceinline__ void init(const UmmaArgs& a, int m0, int kbeg) {
-    const int tid = threadIdx.x, hw = a.H * a.W;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int m = m0 + (2 * i + (tid >> 6)) * 8 + (tid & 7);
-      if (m < a.M) {
-        const int b = m / hw, rem = m - b * hw;
-        bimg[i] = b * hw;
-        yx[i] = ((rem / a.W) << 16) | (rem % a.W);
-      } else {
-        bimg[i] = -1;
-        yx[i] = 0;
-      }
+  const __nv_bfloat16* row[4];  // CONV: the row's pixel in X1, channel 0
+  uint32_t mask[4];             // CONV: tap_mask of the row's pixel (0 beyond the batch)
+  int pix[4];                   // CONV: the pixel's index
+  int tap, ci;                  // CONV: of the thread's K group in the next chunk; WGRAD: of its group (ci < 0: beyond M)
+  int off;                      // WGRAD: element offset of the group from the pixel's channel 0 in X1
+  const __nv_bfloat16* wrow;    // CONV: weights of the thread's first B row at its K group
+  __device__ __forceinline__ void init(const UmmaArgs& a, int m0, int n0, int kbeg) {
+    const int tid = threadIdx.x;
+    const int cin = a.C1 + a.C2;
+    if (a.mode == 5) {
+      const int m = m0 + (tid & 15) * 8;
+      tap = m / cin;
+      ci = m < a.M ? m - tap * cin : -1;
+      const int dy = tap / 3 - 1, dx = tap - 3 * dy - 4;
+      off = (dy * a.W + dx) * a.C1 + ci;
+      return;
     }
-    const int cin = a.C1 + a.C2, k = kbeg + ((tid >> 3) & 7) * 8;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = m0 + (tid >> 3) + 32 * i;
+      mask[i] = 0;
+      pix[i] = 0;
+      if (m < a.M) {
+        const int b = kw_divu(m, a.dhw), rem = m - b * a.H * a.W, y = kw_divu(rem, a.dw);
+        mask[i] = tap_mask(a, y, rem - y * a.W);
+        pix[i] = m;
+      }
+      row[i] = a.X1 + (long long)pix[i] * a.C1;
+    }
+    const int k = kbeg + (tid & 7) * 8;
     tap = k / cin;
     ci = k - tap * cin;
-  }
-  __device__ __forceinline__ void advance(int cin) {
-    ci += kBK;
-    while (ci >= cin) {
-      ci -= cin;
-      ++tap;
-    }
+    wrow = a.Wt + (long long)(n0 + (tid >> 3)) * a.K + (tid & 7) * 8;
   }
 };
 
-// Fill stage tiles for K chunk k0 (all 128 threads).
+// Fill stage tiles for K chunk k0 (all gather threads): asynchronous copies,
+// the caller attaches them to the stage's barrier.
 __device__ __forceinline__ void fill_stage(const UmmaArgs& a, unsigned char* sA, unsigned char* sB, int m0, int n0,
                                            int k0, ConvRows& cr) {
   const int tid = threadIdx.x;
-  if (a.mode == 5) {
-    // weight gradient on MN-major tiles: m = (tap, input channel), n = output
-    // channel, k = pixel; A(p, m) = input[p + tap][ci], B(p, n) = dz[p][co]:
-    // both 8-wide groups are 16 contiguous bytes of the NHWC tensors, copied
-    // as they are (chunk layout as in mode 4)
-    const int k = tid & 63;
-    const int p = k0 + k;
-    const bool pin = p < a.K;
-    int bimg = 0, y = 0, x = 0;
-    if (pin) {
-      const int hw = a.H * a.W;
-      const int b = p / hw, rem = p - b * hw;
-      bimg = b * hw;
-      y = rem / a.W;
-      x = rem - y * a.W;
-    }
-    const int cin = a.C1 + a.C2;
+  if (a.mode == 5 || a.mode == 4) {
+    // MN-major tiles, rows of 8 consecutive m (n) at one k.  Mode 4: A[k][m],
+    // B[k][n] row-major.  Mode 5, weight gradient: m = (tap, input channel),
+    // n = output channel, k = pixel; A(p, m) = input[p + tap][ci], B(p, n) =
+    // dz[p][co], both 16 contiguous bytes of the NHWC tensors
+    unsigned char* ap = sA + (tid & 8 ? kBlock : 0u);
+    if (a.mode == 5 && a.W % kBK == 0) {
+      // the chunk's 64 pixels lie in one image row: one decomposition for all (32 -> 32
+      // channels at 16 x 256^2: 161 us against 242 with one per pixel)
+      const int b = kw_divu(k0, a.dhw), rem = k0 - b * a.H * a.W, y0 = kw_divu(rem, a.dw), x0 = rem - y0 * a.W;
+      const int dy = cr.tap / 3 - 1, dx = cr.tap - 3 * dy - 4, k = tid >> 4;
+      const bool row = cr.ci >= 0 && (unsigned)(y0 + dy) < (unsigned)a.H;
+      const int x = x0 + k + dx;
+      const bool first = cr.ci < a.C1;
+      const __nv_bfloat16* src =
+          !row ? a.X1 : first ? a.X1 + (long long)(k0 + k) * a.C1 + cr.off
+                              : a.X2 + (long long)(b * (a.H >> 1) + ((y0 + dy) >> 1)) * (a.W >> 1) * a.C2 + (cr.ci - a.C1);
 #pragma unroll
-    for (int it = 0; it < 8; ++it) {
-      const int g = it * 2 + (tid >> 6);
-      const int m = m0 + g * 8;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (pin && m < a.M) {
-        const int tap = m / cin;
-        v = conv_chunk_at(a, bimg, y, x, tap, m - tap * cin);
+      for (int i = 0; i < 4; ++i) {
+        const bool in = row && (unsigned)(x + 16 * i) < (unsigned)a.W;
+        cp16_l1(ap + piece_off(k + 16 * i, tid & 7), !in ? a.X1 : src + (first ? 16 * i * a.C1 : ((x + 16 * i) >> 1) * a.C2), in);
       }
-      *reinterpret_cast<uint4*>(sA + g * 1024 + (k >> 3) * 128 + (k & 7) * 16) = v;
-    }
-    for (int c = tid; c < a.NT * 8; c += kThreads) {
-      const int kk = c & 63, g = c >> 6;
-      const int n = n0 + g * 8, pp = k0 + kk;
-      const uint4 v = (n < a.N && pp < a.K) ? ldg16(a.dZ + (long long)pp * a.N + n) : make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(sB + g * 1024 + (kk >> 3) * 128 + (kk & 7) * 16) = v;
-    }
-    return;
-  }
-  if (a.mode == 4) {
-    // MN-major tiles: A[k][m], B[k][n] row-major; chunk (8-row group g of M or N,
-    // k) = 8 consecutive m (n) at one k, stored at g * 1024 + (k / 8) * 128 + (k % 8) * 16
+    } else {
 #pragma unroll
-    for (int it = 0; it < 8; ++it) {
-      const int c = it * kThreads + tid;
-      const int k = c & 63, g = c >> 6;
-      const int m = m0 + g * 8, kk = k0 + k;
-      const uint4 v = (m < a.M && kk < a.K) ? ldg16(a.A + (long long)kk * a.M + m) : make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(sA + g * 1024 + (k >> 3) * 128 + (k & 7) * 16) = v;
-    }
-    for (int c = tid; c < a.NT * 8; c += kThreads) {
-      const int k = c & 63, g = c >> 6;
-      const int n = n0 + g * 8, kk = k0 + k;
-      const uint4 v = (n < a.N && kk < a.K) ? ldg16(a.B + (long long)kk * a.N + n) : make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(sB + g * 1024 + (k >> 3) * 128 + (k & 7) * 16) = v;
-    }
-    return;
-  }
-  if (a.mode == 2) {
-    // WGRAD: A(co, p) = dZ[p][co], B((tap, ci), p) = input[p + tap][ci]; 8 x 8 blocks transposed
-    {
-      const int cb = tid >> 3, pb = tid & 7;  // 16 channel blocks x 8 pixel blocks
-      uint4 in[8], out[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int p = k0 + pb * 8 + j;
-        const int co = m0 + cb * 8;
-        in[j] = (p < a.K && co < a.M) ? ldg16(a.dZ + (long long)p * a.M + co) : make_uint4(0, 0, 0, 0);
-      }
-      transpose8(in, out);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(sA + chunk_off(cb * 8 + i, pb)) = out[i];
-    }
-    const int nblk = (a.NT >> 3) * 8;
-    const int cin = a.C1 + a.C2, hw = a.H * a.W;
-    for (int q = tid; q < nblk; q += kThreads) {
-      const int nb8 = q >> 3, pb = q & 7;
-      const int n = n0 + nb8 * 8;
-      const int tap = n / cin, ci = n - tap * cin;
-      // the block's 8 consecutive pixels, walked from the first without divisions
-      const int p0 = k0 + pb * 8;
-      int b = p0 / hw, rem = p0 - b * hw;
-      int y = rem / a.W, x = rem - y * a.W;
-      uint4 in[8], out[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        in[j] = (p0 + j < a.K && n < a.N) ? conv_chunk_at(a, b * hw, y, x, tap, ci) : make_uint4(0, 0, 0, 0);
-        if (++x == a.W) {
-          x = 0;
-          if (++y == a.H) {
-            y = 0;
-            ++b;
-          }
+      for (int i = 0; i < 4; ++i) {
+        const int k = (tid >> 4) + 16 * i, p = k0 + k;
+        const __nv_bfloat16* src = a.mode == 5 ? a.X1 : a.A;
+        bool in = p < a.K;
+        if (a.mode == 5) {
+          const int pp = in ? p : 0;
+          const int b = kw_divu(pp, a.dhw), rem = pp - b * a.H * a.W;
+          const int y = kw_divu(rem, a.dw), x = rem - y * a.W;
+          in = in && cr.ci >= 0 && ((tap_mask(a, y, x) >> cr.tap) & 1u);
+          if (in) src = cr.ci < a.C1 ? a.X1 + (long long)pp * a.C1 + cr.off : conv_src(a, b, y, x, cr.tap, cr.ci);
+        } else {
+          const int m = m0 + (tid & 15) * 8;
+          in = in && m < a.M;
+          if (in) src += (long long)p * a.M + m;
         }
+        cp16_l1(ap + piece_off(k, tid & 7), src, in);
       }
-      transpose8(in, out);
+    }
+    const __nv_bfloat16* Bm = a.mode == 5 ? a.dZ : a.B;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(sB + chunk_off(nb8 * 8 + i, pb)) = out[i];
+    for (int i = 0; i < 2; ++i) {
+      const int k = (tid >> 3) + 32 * i, p = k0 + k;
+      const __nv_bfloat16* bp = Bm + (long long)p * a.N + n0 + (tid & 7) * 8;
+      for (int j = 0; 64 * j < a.NT; ++j) {
+        const int nn = 64 * j + (tid & 7) * 8;  // within the tile
+        if (nn >= a.NT) break;
+        const bool in = p < a.K && n0 + nn < a.N;
+        cp16(sB + j * kBlock + piece_off(k, tid & 7), in ? bp + 64 * j : Bm, in);
+      }
     }
     return;
   }
-  // GEMM / CONV: A rows are output rows (pixels), 8 K groups of 8 per row;
-  // this thread's group is kc, its rows those of ConvRows
-  const int kc = (tid >> 3) & 7;
+  // GEMM / CONV: rows of 64 k; this thread's group is kc, its rows rr + 32 i
+  const int kc = tid & 7, k = k0 + kc * 8, rr = tid >> 3;
+  const uint32_t at = piece_off(rr, kc);
   if (a.mode == 0) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = (2 * i + (tid >> 6)) * 8 + (tid & 7);
-      const int m = m0 + r, k = k0 + kc * 8;
-      const uint4 v = (m < a.M && k < a.K) ? ldg16(a.A + (long long)m * a.K + k) : make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(sA + chunk_off(r, kc)) = v;
+    for (int i = 0; i < 4; ++i) {
+      const int m = m0 + rr + 32 * i;
+      const bool in = m < a.M && k < a.K;
+      cp16(sA + at + i * 4096, in ? a.A + (long long)m * a.K + k : a.A, in);
     }
-  } else {
-    uint4 v[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      v[i] = cr.bimg[i] < 0 ? make_uint4(0, 0, 0, 0)
-                            : conv_chunk_at(a, cr.bimg[i], cr.yx[i] >> 16, cr.yx[i] & 0xFFFF, cr.tap, cr.ci);
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      *reinterpret_cast<uint4*>(sA + chunk_off((2 * i + (tid >> 6)) * 8 + (tid & 7), kc)) = v[i];
-    cr.advance(a.C1 + a.C2);
+    for (int i = 0; rr + 32 * i < a.NT; ++i) {
+      const int n = n0 + rr + 32 * i;
+      const bool in = n < a.N && k < a.K;
+      cp16(sB + at + i * 4096, in ? a.B + (long long)n * a.K + k : a.B, in);
+    }
+    return;
   }
-  const __nv_bfloat16* Bm = a.mode == 0 ? a.B : a.Wt;
-  for (int c = tid; c < a.NT * 8; c += kThreads) {
-    const int r = (c >> 6) * 8 + (c & 7), kc = (c >> 3) & 7;
-    const int n = n0 + r, k = k0 + kc * 8;
-    const uint4 v = (n < a.N && k < a.K) ? ldg16(Bm + (long long)n * a.K + k) : make_uint4(0, 0, 0, 0);
-    *reinterpret_cast<uint4*>(sB + chunk_off(r, kc)) = v;
+  const int dy = cr.tap / 3 - 1, dx = cr.tap - 3 * dy - 4;
+  const bool first = cr.ci < a.C1;
+  const int off = (dy * a.W + dx) * a.C1 + cr.ci;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const bool in = cr.tap < 9 && ((cr.mask[i] >> cr.tap) & 1u);
+    const __nv_bfloat16* src = a.X1;
+    if (in) {
+      if (first) {
+        src = cr.row[i] + off;
+      } else {
+        const int b = kw_divu(cr.pix[i], a.dhw), rem = cr.pix[i] - b * a.H * a.W, y = kw_divu(rem, a.dw);
+        src = conv_src(a, b, y, rem - y * a.W, cr.tap, cr.ci);
+      }
+    }
+    cp16_l1(sA + at + i * 4096, src, in);
+  }
+  cr.ci += kBK;
+  while (cr.ci >= a.C1 + a.C2) {
+    cr.ci -= a.C1 + a.C2;
+    ++cr.tap;
+  }
+  const __nv_bfloat16* wp = cr.wrow + k0;
+  const long long step = 32LL * a.K;
+  const int nb = k < a.K ? a.N - n0 - rr : 0;  // rows from the thread's first on
+  for (int i = 0; rr + 32 * i < a.NT; ++i, wp += step) {
+    const bool in = 32 * i < nb;
+    cp16(sB + at + i * 4096, in ? wp : a.Wt, in);
   }
 }
 
 // Fill a halo stage: A halo of channels ci0..ci0+15 around pixels (y, x0..x0+127)
-// of image bimg, and the 9 taps x NT output channels of weights for them.
-__device__ __forceinline__ void fill_halo(const UmmaArgs& a, unsigned char* sA, unsigned char* sB, int bimg, int y,
+// of image b, and the 9 taps x NT output channels of weights for them.
+__device__ __forceinline__ void fill_halo(const UmmaArgs& a, unsigned char* sA, unsigned char* sB, int b, int y,
                                           int x0, int n0, int ci0) {
   const int tid = threadIdx.x;
   for (int q = tid; q < 2 * 3 * kHaloCols; q += kThreads) {
     const int kg = q / (3 * kHaloCols), rem = q - kg * (3 * kHaloCols);
     const int r = rem / kHaloCols, col = rem - r * kHaloCols;
     const int yy = y + r - 1, xx = x0 + col - 1, ci = ci0 + kg * 8;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (yy >= 0 && yy < a.H && xx >= 0 && xx < a.W) {
-      if (ci < a.C1)
-        v = ldg16(a.X1 + ((long long)bimg + yy * a.W + xx) * a.C1 + ci);
-      else
-        v = ldg16(a.X2 + ((long long)(bimg >> 2) + (yy >> 1) * (a.W >> 1) + (xx >> 1)) * a.C2 + (ci - a.C1));
-    }
-    *reinterpret_cast<uint4*>(sA + kg * kHaloGroup + rem * 16) = v;
+    const bool in = (unsigned)yy < (unsigned)a.H && (unsigned)xx < (unsigned)a.W;
+    cp16_l1(sA + kg * kHaloGroup + rem * 16, in ? conv_src(a, b, yy, xx, 4, ci) : a.X1, in);
   }
   const int cin = a.C1 + a.C2;
   for (int q = tid; q < 18 * a.NT; q += kThreads) {
     const int kg = q & 1, nt = q >> 1;
     const int n = nt / 9, tap = nt - n * 9;
-    const uint4 v = (n0 + n < a.N) ? ldg16(a.Wt + ((long long)(n0 + n) * 9 + tap) * cin + ci0 + kg * 8)
-                                   : make_uint4(0, 0, 0, 0);
-    *reinterpret_cast<uint4*>(sB + ((tap * 2 + kg) * a.NT + n) * 16) = v;
+    const bool in = n0 + n < a.N;
+    cp16(sB + ((tap * 2 + kg) * a.NT + n) * 16, in ? a.Wt + ((long long)(n0 + n) * 9 + tap) * cin + ci0 + kg * 8 : a.Wt, in);
   }
 }
 
-__global__ void __launch_bounds__(kThreads) k_umma(UmmaArgs a, int* err) {
+// TMEM columns of one accumulator of NT columns, and accumulators per tile: two
+// for the weight gradients, whose sums run over thousands of pixels (the error
+// of the tensor core's accumulation grows with the chain: 8e-6 relative with 648
+// MMAs in one, 4e-6 in two of 324), added in the epilogue.
+__host__ __device__ constexpr uint32_t acc_cols(int NT) { return NT <= 32 ? 32u : NT <= 64 ? 64u : NT <= 128 ? 128u : 256u; }
+__host__ __device__ constexpr uint32_t acc_count(int mode) { return mode == 5 ? 2u : 1u; }
+
+__global__ void __launch_bounds__(kThreads + 32, 2) k_umma(const __grid_constant__ UmmaArgs a, int* err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  // stage s: A at base + s astage, B at base + 2 astage + s bstage
+  // stage s: A at base + s astage, B at base + S astage + s bstage
   const bool halo = a.mode == 3;
+  const int S = a.stages;
   const uint32_t astage = halo ? kAHalo : (uint32_t)kATile;
-  const uint32_t bstage = halo ? (uint32_t)a.NT * 288u : (uint32_t)a.NT * (kBK * 2);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(base + 2 * astage + 2 * bstage);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
-  __shared__ int s_fail;
+  // MN-major tiles (modes 4, 5) keep whole 64-wide blocks
+  const bool mn = a.mode == 4 || a.mode == 5;
+  const uint32_t bstage = halo ? (uint32_t)a.NT * 288u : mn ? (uint32_t)(a.NT + 63) / 64 * kBlock : (uint32_t)a.NT * (kBK * 2);
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + S * (astage + bstage));
+  uint64_t* empty = full + kMaxStages;
+  uint64_t* done = empty + kMaxStages;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
+  __shared__ volatile int s_fail;
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * a.NT;
-  const uint32_t ncols = a.NT <= 32 ? 32 : a.NT <= 64 ? 64 : a.NT <= 128 ? 128 : 256;
+  // the tile's products go to nacc accumulators of `acols` columns in turn
+  const uint32_t acols = acc_cols(a.NT), nacc = acc_count(a.mode), ncols = acols * nacc;
   if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
+    for (int i = 0; i < S; ++i) {
+      mbar_init(&full[i], kThreads);
+      mbar_init(&empty[i], 1);
+    }
+    mbar_init(done, 1);
     s_fail = 0;
     kwtma::fence_barrier_init();
   }
@@ -444,45 +462,51 @@ __global__ void __launch_bounds__(kThreads) k_umma(UmmaArgs a, int* err) {
   const uint32_t tmem = *tslot;
 
   int kbeg = 0, kend = a.K;
-  if (a.mode == 2 || a.mode == 5 || (a.mode == 1 && a.ksplit > 0)) {
+  if (a.mode == 5 || (a.mode == 1 && a.ksplit > 0)) {
     kbeg = blockIdx.z * a.ksplit;
     kend = min(a.K, kbeg + a.ksplit);
   }
   const int nchunks = halo ? (a.C1 + a.C2) / 16 : (kend - kbeg + kBK - 1) / kBK;
-  // MN-major tiles (modes 4, 5): 8-element groups along M / N 1024 bytes apart
-  // (SBO), K core matrices 128 bytes apart (LBO), as in the K-major layout
-  const bool mn = a.mode == 4 || a.mode == 5;
-  const uint32_t idesc = mn ? idesc_bf16_mn(kBM, a.NT) : idesc_bf16(kBM, a.NT);
-  int hb = 0, hy = 0, hx = 0;  // halo tiles: image, row and first column of the tile
-  if (halo) {
-    const int hw = a.H * a.W;
-    hb = (m0 / hw) * hw;
-    hy = (m0 - hb) / a.W;
-    hx = m0 - hb - hy * a.W;
-  }
-  ConvRows cr;
-  if (a.mode == 1) cr.init(a, m0, kbeg);
-  bool ok = true;
-  for (int c = 0; c < nchunks && ok; ++c) {
-    const int s = c & 1;
-    if (c >= 2) {
-      if (!mbar_wait(&bar[s], ((c - 2) >> 1) & 1, kWaitNs)) ok = false;
-      if (__syncthreads_or(!ok)) {
-        ok = false;
-        break;
+  if (warp < kThreads / 32) {
+    // ---------------- gather ----------------
+    int hb = 0, hy = 0, hx = 0;  // halo tiles: image, row and first column of the tile
+    if (halo) {
+      const int hw = a.H * a.W;
+      hb = m0 / hw;
+      hy = (m0 - hb * hw) / a.W;
+      hx = m0 - hb * hw - hy * a.W;
+    }
+    ConvRows cr;
+    if (a.mode == 1 || a.mode == 5) cr.init(a, m0, n0, kbeg);
+    int s = 0, phase = 1;  // stage of chunk c, parity of its last release
+    for (int c = 0; c < nchunks; ++c) {
+      if (c >= S && !mbar_wait(&empty[s], phase, kWaitNs)) s_fail = 1;
+      if (s_fail) break;
+      unsigned char* sA = base + s * astage;
+      unsigned char* sB = base + S * astage + s * bstage;
+      if (halo)
+        fill_halo(a, sA, sB, hb, hy, hx, n0, c * 16);
+      else
+        fill_stage(a, sA, sB, m0, n0, kbeg + c * kBK, cr);
+      cp_arrive(&full[s]);
+      if (++s == S) {
+        s = 0;
+        phase ^= 1;
       }
     }
-    unsigned char* sAs = base + s * astage;
-    unsigned char* sBs = base + 2 * astage + s * bstage;
-    if (halo)
-      fill_halo(a, sAs, sBs, hb, hy, hx, n0, c * 16);
-    else
-      fill_stage(a, sAs, sBs, m0, n0, kbeg + c * kBK, cr);
-    fence_async_smem();
-    __syncthreads();
-    if (tid == 0) {
+    cp_wait_all();
+  } else if (lane == 0) {
+    // ---------------- tensor cores ----------------
+    const uint32_t idesc = mn ? idesc_bf16_mn(kBM, a.NT) : idesc_bf16(kBM, a.NT);
+    int s = 0, phase = 0;
+    for (int c = 0; c < nchunks; ++c) {
+      if (!mbar_wait(&full[s], phase, kWaitNs)) s_fail = 1;
+      if (s_fail) break;
+      // the copies, seen through the barrier, before the tensor cores' reads: fenced
+      // here once, since a fence in the gatherers would drain their copies in flight
+      fence_async_smem();
       tc_fence_after();
-      const uint32_t ab = smem_u32(sAs), bb = smem_u32(sBs);
+      const uint32_t ab = smem_u32(base + s * astage), bb = smem_u32(base + S * astage + s * bstage);
       if (halo) {
         // tap (dy, dx): the halo from row 1 + dy, column 1 + dx; the tap's weights
 #pragma unroll
@@ -494,30 +518,41 @@ __global__ void __launch_bounds__(kThreads) k_umma(UmmaArgs a, int* err) {
       } else if (mn) {
 #pragma unroll
         for (int kk = 0; kk < kBK / 16; ++kk)
-          umma_bf16(tmem, smem_desc(ab + kk * 256, 128, 1024), smem_desc(bb + kk * 256, 128, 1024), idesc,
-                    (c | kk) != 0);
+          umma_bf16(tmem + ((4 * c + kk) & (nacc - 1)) * acols, smem_desc_mn128(ab + kk * 2048, kBlock),
+                    smem_desc_mn128(bb + kk * 2048, kBlock), idesc, 4 * c + kk >= (int)nacc);
       } else {
 #pragma unroll
         for (int kk = 0; kk < kBK / 16; ++kk)
-          umma_bf16(tmem, smem_desc(ab + kk * 2 * kLBO), smem_desc(bb + kk * 2 * kLBO), idesc, (c | kk) != 0);
+          umma_bf16(tmem + ((4 * c + kk) & (nacc - 1)) * acols, smem_desc_k128(ab + kk * 32),
+                    smem_desc_k128(bb + kk * 32), idesc, 4 * c + kk >= (int)nacc);
       }
-      umma_commit(&bar[s]);
+      umma_commit(&empty[s]);
+      if (++s == S) {
+        s = 0;
+        phase ^= 1;
+      }
     }
+    // every MMA issued has completed before the accumulator is read and freed
+    umma_commit(done);
+    if (!mbar_wait(done, 0, kWaitNs)) s_fail = 1;
   }
-  if (ok && nchunks > 0) {
-    const int L = nchunks - 1;
-    if (!mbar_wait(&bar[L & 1], (L >> 1) & 1, kWaitNs)) ok = false;
-  }
-  if (!ok) s_fail = 1;
   __syncthreads();
   tc_fence_after();
-  if (!s_fail && nchunks > 0) {
-    const int r = warp * 32 + (tid & 31);
+  if (!s_fail && nchunks > 0 && warp < 8) {
+    const int r = (warp & 3) * 32 + lane;
     const int m = m0 + r;
-    const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-    for (int j0 = 0; j0 < a.NT; j0 += 16) {
+    const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t used = min(nacc, 4u * (uint32_t)nchunks);  // accumulators written
+    for (int j0 = (warp >> 2) * 16; j0 < a.NT; j0 += 32) {
       float v[16];
+      __syncwarp();
       tmem_ld16(trow + (uint32_t)j0, v);
+      for (uint32_t q = 1; q < used; ++q) {
+        float u[16];
+        tmem_ld16(trow + q * acols + (uint32_t)j0, u);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] += u[j];
+      }
       if (m >= a.M) continue;
       if (a.mode == 0 || a.mode == 4) {
 #pragma unroll
@@ -568,13 +603,6 @@ __global__ void __launch_bounds__(kThreads) k_umma(UmmaArgs a, int* err) {
         for (int j = 0; j < 16; ++j) {
           const int n = n0 + j0 + j;
           if (n < a.N) atomicAdd(a.dW + (long long)n * a.M + m, v[j]);
-        }
-      } else {
-        // WGRAD: add this pixel range's partial tile
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int n = n0 + j0 + j;
-          if (n < a.N) atomicAdd(a.dW + (long long)m * a.N + n, v[j]);
         }
       }
     }
@@ -1064,13 +1092,24 @@ int g_umma_attr_dev = -1;
 
 int umma_fail(int code, const char* msg) { return kw_internal_fail(code, msg); }
 
-// Dynamic shared memory of a launch: the two A stages, two B stages of the
-// launch's tile width, barriers and alignment slack -- at least enough that no
-// more CTAs share an SM than its 512 TMEM columns hold (256-column tiles: 2
-// CTAs, 128-column tiles: 4), so that tcgen05.alloc never has to wait.
-int umma_smem(int NT, bool halo = false) {
-  const int need = halo ? 2 * (int)kAHalo + 2 * NT * 288 + 64 + 1024 : 2 * kATile + 2 * NT * kBK * 2 + 64 + 1024;
-  const int ncols = NT <= 32 ? 32 : NT <= 64 ? 64 : NT <= 128 ? 128 : 256;
+// Ring depth of a launch: as deep as two CTAs fit an SM's shared memory, or,
+// where that leaves fewer than three stages, one CTA.
+int umma_stage_bytes(int NT, int mode) {
+  return mode == 3 ? (int)kAHalo + NT * 288 : kATile + (mode >= 4 ? (NT + 63) / 64 * (int)kBlock : NT * kBK * 2);
+}
+int umma_stages(int NT, int mode) {
+  const int b = umma_stage_bytes(NT, mode);
+  const int two = 108 * 1024 / b, one = 220 * 1024 / b;
+  return std::min(kMaxStages, two >= 3 ? two : one);
+}
+
+// Dynamic shared memory of a launch: the stages, barriers and alignment slack
+// -- at least enough that no more CTAs share an SM than its 512 TMEM columns
+// hold (256-column tiles: 2 CTAs, 128-column tiles: 4), so that tcgen05.alloc
+// never has to wait.
+int umma_smem(int NT, int mode) {
+  const int need = umma_stages(NT, mode) * umma_stage_bytes(NT, mode) + 128 + 1024;
+  const int ncols = (int)(acc_cols(NT) * acc_count(mode));
   const int floor_bytes = ncols == 256 ? 80 * 1024 : ncols == 128 ? 48 * 1024 : 0;
   return need > floor_bytes ? need : floor_bytes;
 }
@@ -1078,14 +1117,21 @@ int umma_smem(int NT, bool halo = false) {
 int umma_launch(UmmaArgs& a, dim3 grid, cudaStream_t st) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return umma_fail(KW_ERR_CUDA, "cudaGetDevice failed");
-  const int smem = umma_smem(a.NT, a.mode == 3);
+  const int smem = umma_smem(a.NT, a.mode);
+  a.stages = umma_stages(a.NT, a.mode);
+  if (a.H > 0) {
+    a.dhw = kw_divu_make((uint32_t)(a.H * a.W));
+    a.dw = kw_divu_make((uint32_t)a.W);
+  }
   if (g_umma_attr_dev != dev) {
-    const int most = std::max(umma_smem(kMaxNT), umma_smem(kMaxNT, true));
+    int most = 0;
+    for (int nt = 16; nt <= kMaxNT; nt += 16)
+      for (int mode : {0, 3, 4}) most = std::max(most, umma_smem(nt, mode));
     if (cudaFuncSetAttribute(k_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
       return umma_fail(KW_ERR_CUDA, "k_umma: cannot set the shared-memory size");
     g_umma_attr_dev = dev;
   }
-  k_umma<<<grid, kThreads, smem, st>>>(a, kw_device_error_ptr());
+  k_umma<<<grid, kThreads + 32, smem, st>>>(a, kw_device_error_ptr());
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     char buf[256];
@@ -1095,9 +1141,16 @@ int umma_launch(UmmaArgs& a, dim3 grid, cudaStream_t st) {
   return KW_OK;
 }
 
-int tile_cols(int n) {
-  const int r = (n + 15) / 16 * 16;
-  return r > kMaxNT ? kMaxNT : r;
+// Tile columns for n output columns and mtile row tiles: the fewest tiles of at
+// most `cap`, of equal width; halved (down to 64) while the grid leaves SMs idle.
+int tile_cols(int n, long long mtile = 1LL << 40, int nsm = 0, int cap = kMaxNT) {
+  int nt = (n + cap - 1) / cap;
+  int c = ((n + nt - 1) / nt + 15) / 16 * 16;
+  while (c > 64 && nt * mtile < nsm) {
+    nt *= 2;
+    c = ((n + nt - 1) / nt + 15) / 16 * 16;
+  }
+  return c;
 }
 
 // --- persistent TMA-fed convolution (k_conv_tma) ---------------------------
@@ -1289,16 +1342,22 @@ int32_t kw_conv3x3(const void* x1, int32_t c1, const void* x2, int32_t c2, int32
     const int rc = conv_tma_try(a, st);
     if (rc != 1) return rc;
   }
-  const int ntile = (cout + a.NT - 1) / a.NT, mtile = (a.M + kBM - 1) / kBM;
+  // wide outputs fill the gather tiles' tensor time better than the halo saves
+  // loads (64 -> 192 channels at 16 x 128^2: 211 us against 253; 96 -> 64: 209
+  // either way; 96 -> 32 at 16 x 256^2: 465 against 338)
+  if (a.NT > 128) a.mode = 1;
+  const int mtile = (a.M + kBM - 1) / kBM;
   // gather tiles that leave SMs idle (small images, many channels): the K
   // range is split over CTAs whose partial tiles are added in f32 scratch,
   // then bias, ReLU and the stores run as one elementwise pass
   int dev = 0, nsm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return umma_fail(KW_ERR_CUDA, "kw_conv3x3: device query failed");
+  if (a.mode == 1) a.NT = tile_cols(cout, mtile, nsm);
+  const int ntile = (cout + a.NT - 1) / a.NT;
   const int nchunk = (a.K + kBK - 1) / kBK;
   int split = 1;
-  if (a.mode == 1 && ntile * mtile < nsm) split = std::min((2 * nsm + ntile * mtile - 1) / (ntile * mtile), nchunk / 2);
+  if (a.mode == 1 && 2 * ntile * mtile < nsm) split = std::min((nsm + ntile * mtile - 1) / (ntile * mtile), nchunk / 4);
   if (split <= 1) return umma_launch(a, dim3(ntile, mtile), st);
   const int per = (nchunk + split - 1) / split;
   split = (nchunk + per - 1) / per;
@@ -1327,24 +1386,19 @@ int32_t kw_conv3x3_wgrad(const void* x1, int32_t c1, const void* x2, int32_t c2,
   if (!x1 || !dz || !dw) return umma_fail(KW_ERR_INVALID, "kw_conv3x3_wgrad: null argument");
   if (c1 <= 0 || c1 % 8 || c2 < 0 || c2 % 8 || (c2 && !x2) || cout <= 0 || cout % 8)
     return umma_fail(KW_ERR_INVALID, "kw_conv3x3_wgrad: channels must be multiples of 8");
-  // MN-major tiles (rows (tap, input channel), columns output channels) unless
-  // KWAVE_GB300_WGRAD_MN=0 selects the transposing K-major tiles
-  static const bool mn_ok = [] {
-    const char* env = getenv("KWAVE_GB300_WGRAD_MN");
-    return !(env && env[0] == '0');
-  }();
+  // MN-major tiles: rows (tap, input channel), columns output channels
   UmmaArgs a;
   memset(&a, 0, sizeof a);
-  a.mode = mn_ok ? 5 : 2;
+  a.mode = 5;
   a.nb = nb;
   a.H = H;
   a.W = W;
   a.C1 = c1;
   a.C2 = c2;
-  a.M = mn_ok ? 9 * (c1 + c2) : cout;
-  a.N = mn_ok ? cout : 9 * (c1 + c2);
+  a.M = 9 * (c1 + c2);
+  a.N = cout;
   a.K = nb * H * W;
-  a.NT = tile_cols(a.N);
+  a.NT = tile_cols(a.N, 1LL << 40, 0, 128);  // two accumulators, two CTAs per SM
   a.X1 = static_cast<const __nv_bfloat16*>(x1);
   a.X2 = static_cast<const __nv_bfloat16*>(x2);
   a.dZ = static_cast<const __nv_bfloat16*>(dz);
@@ -1354,7 +1408,7 @@ int32_t kw_conv3x3_wgrad(const void* x1, int32_t c1, const void* x2, int32_t c2,
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  long long want = 4LL * nsm / (ntile * mtile);
+  long long want = 2LL * nsm / (ntile * mtile);
   if (want < 1) want = 1;
   long long per = ((long long)a.K + want - 1) / want;
   per = (per + kBK - 1) / kBK * kBK;
