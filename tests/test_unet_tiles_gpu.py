@@ -60,3 +60,34 @@ def test_gathered_tiles(nb, H, W, c1, c2, cout):
     e_w = rel(dw.reshape(cout, 3, 3, c1 + c2).permute(0, 3, 1, 2), wt.grad)
     print(f"{nb}x{H}x{W} {c1}+{c2}->{cout}: forward {e_y:.2e} weight gradient {e_w:.2e}")
     assert e_y <= F32_TOL and e_w <= F32_TOL
+
+
+@pytest.mark.parametrize("npix,C", [(1, 8), (77, 24), (1000, 32), (4097, 48), (70000, 8), (513, 2048), (5, 4104)])
+@pytest.mark.parametrize("shift", [0, 1])  # 1: tensors that do not start on 16 bytes
+def test_elementwise_gradients(npix, C, shift):
+    """ReLU and bias gradients, eight values per access and one by one."""
+    import torch
+
+    from kwave_gb300 import unet_ops as U
+
+    n = npix * C
+    dy, y = bf((n + shift,), 6), bf((n + shift,), 7)
+    y[shift::3] = 0.0
+    dz = U.relu_grad(dy.cuda()[shift:], y.cuda()[shift:])
+    db = torch.ones(C, dtype=torch.float32, device="cuda")
+    U.bias_grad(dy.cuda()[shift:].reshape(npix, C), db)
+    torch.cuda.synchronize()
+    assert torch.equal(dz.cpu(), torch.where(y[shift:].float() > 0, dy[shift:], torch.zeros_like(dy[shift:])))
+    ref = dy[shift:].double().reshape(npix, C)
+    e = float((db.cpu().double() - 1 - ref.sum(0)).norm() / (1 + ref.abs().sum(0)).norm())
+    assert e <= F32_TOL
+
+
+@pytest.mark.parametrize("cout,cin", [(8, 8), (32, 32), (40, 72), (256, 8)])
+def test_flipped_weights(cout, cin):
+    import torch
+
+    from kwave_gb300 import unet_ops as U
+
+    w = bf((cout, 9, cin), 8)
+    assert torch.equal(U.flip_weights(w.cuda()).cpu(), w.flip(1).permute(2, 1, 0).contiguous())
