@@ -194,8 +194,8 @@ __global__ void k_loop_tick(cudaGraphConditionalHandle h, int* left) {
   cudaGraphSetConditional(h, v > 0 ? 1u : 0u);
 }
 
-__global__ void k_step_tick(int* tdev) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *tdev += 1;
+__global__ void k_step_tick(int* tdev, int steps) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) *tdev += steps;
 }
 
 // ---------------------------------------------------------------------------

@@ -233,7 +233,7 @@ __global__ void k_step_set(int* tdev, int t);
 // out = rho_0 + rho_1 (+ rho_2): the forward density sum, in the step's order
 __global__ void k_density_sum(float* __restrict__ out, const float* __restrict__ r0, const float* __restrict__ r1,
                               const float* __restrict__ r2, long long n);
-__global__ void k_step_tick(int* tdev);
+__global__ void k_step_tick(int* tdev, int steps);
 __global__ void k_loop_set(int* left, int n);
 __global__ void k_loop_tick(cudaGraphConditionalHandle h, int* left);
 __global__ void k_step_tick_group(int* const* tdev, int n);

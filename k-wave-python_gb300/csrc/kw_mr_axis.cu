@@ -48,6 +48,7 @@ cudaError_t kw_mr_axis_plan(const AxisParams& A, const KwMrLen& L, const float2*
   W.ncoltot = (uint32_t)A.ncols * (uint32_t)nouter;
   W.gate = nullptr;
   W.gate_end = 0;
+  W.pdl = 0;
   int nitems = nb, nbuf = 1;
   if (A.mode < 2) {
     X.kind = A.mode == 0 ? MK_FWD : MK_INV;

@@ -20,6 +20,7 @@
 #include "kw_kernels.cuh"
 #include "kw_mr.cuh"
 #include "kw_regfft.cuh"
+#include "kw_tma.cuh"
 
 enum KwMrKind { MK_FWD = 0, MK_INV = 1, MK_GRAD = 2, MK_DIV = 3, MK_NAB = 4, MK_GEN = 5 };
 
@@ -35,6 +36,7 @@ struct MrAxisParams {
   const int* gate;       // grouped source passes: device step counter; the pass is idle from step
   int gate_end;          // gate_end on (null: always on)
   int gx;                // column tiles (grouped launches)
+  int pdl;               // launched as a programmatic dependent (host)
   float nab_inv, nab_fac[2];  // MK_NAB: |k|^2 is scaled by nab_inv (a power of two) before its
                               // logarithm, nab_fac[q] undoes it: |k|^p = 2^(p/2 log2(|k|^2 inv)) fac
 };
@@ -314,6 +316,8 @@ __device__ __forceinline__ void mr_axis_body(const MrAxisParams& W, int tile, in
   const uint32_t c = act ? q - outer * (uint32_t)P.ncols : 0u;
   const uint32_t base = outer * (uint32_t)P.os + c;
   const uint32_t xs = (uint32_t)P.xs;
+  // up to here and in the column's factors only the parameters and the plan's tables are read
+  if constexpr (KIND == MK_FWD || KIND == MK_INV) kwtma::grid_dep_wait();
 
   if constexpr (KIND == MK_FWD) {
     float2* buf = P.bufs[P.plain[item]] + base;
@@ -326,6 +330,7 @@ __device__ __forceinline__ void mr_axis_body(const MrAxisParams& W, int tile, in
     }
     __syncthreads();
     axis_mids<false>(A, L, W.tw, it0, nit, cc, W.lgT);
+    kwtma::grid_dep_launch();
     switch (L.rl) {
 #define KW_MR_CASE(R) \
   case R: axis_last_fwd<R>(A, W, buf, act, it0, nit, cc); break;
@@ -344,6 +349,7 @@ __device__ __forceinline__ void mr_axis_body(const MrAxisParams& W, int tile, in
     }
     __syncthreads();
     axis_mids<true>(A, L, W.tw, it0, nit, cc, W.lgT);
+    kwtma::grid_dep_launch();
     auto store = [&](int row, float2 v) {
       if (act) buf[(uint32_t)row * xs] = v;
     };
@@ -360,6 +366,7 @@ __device__ __forceinline__ void mr_axis_body(const MrAxisParams& W, int tile, in
     const ColK g = col_geometry(P, (int)c);
     const bool on = act && g.valid;
     const float lo = mr_col_lo(P, g);
+    kwtma::grid_dep_wait();
     switch (L.r[0]) {
 #define KW_MR_CASE(R) \
   case R: axis_first_fwd<R>(A, W, in, act, it0, nit, cc); break;
@@ -382,6 +389,7 @@ __device__ __forceinline__ void mr_axis_body(const MrAxisParams& W, int tile, in
       axis_mids<true>(A, L, W.tw, it0, nit, cc, W.lgT);
       if constexpr (KIND == MK_GRAD) {
         axis_mids<true>(B, L, W.tw, it0, nit, cc, W.lgT);
+        kwtma::grid_dep_launch();
         const float2 f1 = mr_col_factor(P, OP_GRAD, 1, g);
         const float2 f2 = P.ndim == 3 ? mr_col_factor(P, OP_GRAD, 2, g) : make_float2(0.f, 0.f);
         float2* o0 = P.bufs[0] + base;
@@ -407,6 +415,7 @@ __device__ __forceinline__ void mr_axis_body(const MrAxisParams& W, int tile, in
           default: break;
         }
       } else {
+        kwtma::grid_dep_launch();
         float2* out = P.bufs[ib] + base;
         auto store = [&](int row, float2 v) {
           if (act) out[(uint32_t)row * xs] = v;
@@ -486,7 +495,7 @@ static cudaError_t kw_mr_axis_go(dim3 grid, int threads, size_t smem, cudaStream
   if (Ps)
     k_mr_axis_group<KIND><<<grid, threads, smem, st>>>(Ps, map);
   else
-    k_mr_axis<KIND><<<grid, threads, smem, st>>>(*W);
+    return kwtma::launch_k(k_mr_axis<KIND>, grid, dim3(threads), smem, st, W->pdl, *W);
   return cudaGetLastError();
 }
 

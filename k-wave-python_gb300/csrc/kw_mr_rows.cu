@@ -32,6 +32,7 @@ void kw_mr_rows_plan(int stage, int nsm, KwMrRowsLaunch& X) {
   int SB = std::max(1, 128 / (nq * P));
   while (SB > 1 && nseq < 4 * nsm * SB) SB = (SB + 1) / 2;
   while (2 * P * SB * nq <= 64 && P < M) P *= 2;
+  W.pdl = 0;
   W.SB = SB;
   W.rpb = odd ? 2 * SB : SB;
   W.P = P;

@@ -24,15 +24,20 @@
 #pragma once
 #include "kw_kernels.cuh"
 #include "kw_mr.cuh"
+#include "kw_tma.cuh"
 
 #define KW_MR_THREADS 192  // most threads of a row block
 #define KW_MR_MAXM 1024    // most points of a sequence
+// Most dynamic shared memory of a row block: one sequence of 1024 points in each
+// of up to six regions, slots of up to 16 / 15 of the points.
+#define KW_MR_ROWS_SMEM (96 * 1024)
 
 struct MrRowsParams {
   RowsParams Q;
   KwMrLen L;
   const float2* tw;       // pass twiddles of the row transform
   const uint32_t* pos;    // slots of frequencies k (low half) and M - k (high half), k < M
+  int pdl;                // launched as a programmatic dependent (host)
   int SB, rpb;            // sequences per region and rows per block
   int P, PT, G;           // threads per sequence (c2r, r2c), per row (physics), sequences at a time: threads / P
   int region;             // slots of a region: SB x L.slots
@@ -189,6 +194,7 @@ struct Rows {
   template <class SPEC>
   __device__ __forceinline__ void r2c(int nq, SPEC spec) const {
     row_passes<false>(A, W.L, nq * W.SB, W.tw);
+    kwtma::grid_dep_launch();
     const int N = W.L.n, P = W.P;
     const int g = kw_divu(threadIdx.x, W.dP), k1 = threadIdx.x - g * P;
 #pragma unroll 1
@@ -380,6 +386,7 @@ __device__ __forceinline__ void mr_rows_body(const MrRowsParams& W, int bx) {
   const Rows<ODD> c(W, bx, reinterpret_cast<float2*>(smem_f4));
   const int D = DIM ? DIM : Q.ndim;
   constexpr int MD = DIM ? DIM : 3;
+  kwtma::grid_dep_wait();
   const int t = kw_step_t(Q);
 
   if constexpr (STAGE == ST_INIT) {
@@ -757,10 +764,13 @@ __global__ void __launch_bounds__(KW_MR_THREADS, kw_mr_blocks(STAGE))
 template <int STAGE, int DIM>
 static cudaError_t kw_mr_rows_go(int odd, int blocks, int threads, size_t smem, cudaStream_t st, const MrRowsParams* W,
                                  const MrRowsParams* Ps, const int2* map) {
+  // one constant, so that plans of several threads never lower it under one another
   if (smem > 40 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_mr_rows<STAGE, true, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > KW_MR_ROWS_SMEM) return cudaErrorInvalidValue;
+    cudaError_t e =
+        cudaFuncSetAttribute(k_mr_rows<STAGE, true, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, KW_MR_ROWS_SMEM);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_mr_rows<STAGE, false, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      e = cudaFuncSetAttribute(k_mr_rows<STAGE, false, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, KW_MR_ROWS_SMEM);
     if (e != cudaSuccess) return e;
   }
   if (Ps) {
@@ -768,7 +778,7 @@ static cudaError_t kw_mr_rows_go(int odd, int blocks, int threads, size_t smem, 
     if constexpr (STAGE == ST_U || STAGE == ST_RHO || STAGE == ST_EOS || STAGE == ST_SRC) {
       if (smem > 40 * 1024) {
         const cudaError_t e =
-            cudaFuncSetAttribute(k_mr_rows_group<STAGE, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            cudaFuncSetAttribute(k_mr_rows_group<STAGE, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, KW_MR_ROWS_SMEM);
         if (e != cudaSuccess) return e;
       }
       k_mr_rows_group<STAGE, DIM><<<blocks, threads, smem, st>>>(Ps, map);
@@ -776,8 +786,8 @@ static cudaError_t kw_mr_rows_go(int odd, int blocks, int threads, size_t smem, 
       return cudaErrorInvalidValue;
     }
   } else if (odd)
-    k_mr_rows<STAGE, true, DIM><<<blocks, threads, smem, st>>>(*W);
+    return kwtma::launch_k(k_mr_rows<STAGE, true, DIM>, dim3(blocks), dim3(threads), smem, st, W->pdl, *W);
   else
-    k_mr_rows<STAGE, false, DIM><<<blocks, threads, smem, st>>>(*W);
+    return kwtma::launch_k(k_mr_rows<STAGE, false, DIM>, dim3(blocks), dim3(threads), smem, st, W->pdl, *W);
   return cudaGetLastError();
 }

@@ -144,6 +144,7 @@ struct kw_plan {
   // step graphs: one captured step per distinct launch sequence, replayed with
   // the step index read from d_tstep
   struct StepGraph {
+    int steps;  // consecutive steps it advances
     int key;
     cudaGraph_t graph;
     cudaGraphExec_t exec;
@@ -155,7 +156,15 @@ struct kw_plan {
   // default: at 256^3 the step took 1.083 ms with it against 1.054 ms without
   // (early CTAs of the next persistent pass land unevenly across SMs).
   bool pdl = false;
+  // Mixed-radix passes launched as programmatic dependents: their blocks start,
+  // read their parameters and work out their place while the pass before drains.
+  // A pass lets the next one start before its last butterflies: 375 x 324 tissue
+  // runs took 60.9 ms without, 57.0 so, and 64.5 with the next pass let in at once
+  // (its blocks then filled up the SMs that had the fewest blocks of this one).
+  // Off for members of batches, whose steps become child graphs.
+  bool mr_pdl = true;
   bool capturing = false;
+  int cap_t0 = 0;  // first step of the steps being captured
   int* d_tstep = nullptr;
   int tstep_val = -1;  // value d_tstep holds once the stream reaches the last enqueued work
   cudaStream_t cap_stream = nullptr;
@@ -181,6 +190,7 @@ struct kw_plan {
 // TMA passes start their prologue while the previous kernel drains, except
 // while every launch is bracketed by timing events.
 static int pdl_ok(const kw_plan* p) { return p->pdl && !p->timing; }
+static int mr_pdl_ok(const kw_plan* p) { return p->mr_pdl && !p->timing && !p->rec_list; }
 
 // Bracket a launch with events when timing is on.
 static int ev_begin(kw_plan* p, cudaStream_t st, size_t* slot) {
@@ -995,8 +1005,8 @@ static int launch_rows(kw_plan* p, int stage, int init, int t, int write_p, cuda
   if (p->capturing) {
     // replayed for other steps: the step index comes from the device counter
     P.tdev = p->d_tstep;
-    P.t = 0;
-    P.rec_row = (t >= p->g.record_start) ? -p->g.record_start : -(1 << 30);
+    P.t = t - p->cap_t0;
+    P.rec_row = (t >= p->g.record_start) ? P.t - p->g.record_start : -(1 << 30);
   }
   P.write_p = write_p;
   P.srcp_on = p->srcp_on;
@@ -1028,6 +1038,7 @@ static int launch_rows(kw_plan* p, int stage, int init, int t, int write_p, cuda
   int rc = ev_begin(p, st, &slot);
   if (rc) return rc;
   if (mr) {
+    X.W.pdl = mr_pdl_ok(p);
     CK(kw_mr_rows_launch(X, st));
   } else if (p->rows_reg && (stage < ST_ADJ_A || adjoint_rows_reg())) {
     P.R = p->rows_R;
@@ -1116,6 +1127,7 @@ static int launch_axis_plain(kw_plan* p, int axis, int inv, const int* bufs, int
   int rc = ev_begin(p, st, &slot);
   if (rc) return rc;
   if (p->axis_mr[axis]) {
+    X.W.pdl = mr_pdl_ok(p);
     CK(kw_mr_axis_launch(X, st));
   } else if (p->tma_axis[axis]) {
     CK(kw_tma_launch(p->tma, axis, p->N[axis], nouter, nb, p->nsm, st, A, pdl_ok(p)));
@@ -1190,6 +1202,7 @@ static int launch_axis_ops(kw_plan* p, const AxisJob* jobs, int nj, cudaStream_t
   int rc = ev_begin(p, st, &slot);
   if (rc) return rc;
   if (p->axis_mr[0]) {
+    X.W.pdl = mr_pdl_ok(p);
     CK(kw_mr_axis_launch(X, st));
   } else if (p->tma_axis[0]) {
     CK(kw_tma_launch(p->tma, 0, p->N[0], 1, 0, p->nsm, st, A, pdl_ok(p)));
@@ -1355,11 +1368,11 @@ static void drop_graphs(kw_plan* p) {
   p->graphs.clear();
 }
 
-// Captured step graph for the key of step t (captured on first use).
-static int step_graph(kw_plan* p, int t, kw_plan::StepGraph** out) {
+// Captured graph of `steps` consecutive steps with the key of step t (captured on first use).
+static int step_graph(kw_plan* p, int t, int steps, kw_plan::StepGraph** out) {
   const int key = step_key(p, t);
   for (auto& g : p->graphs)
-    if (g.key == key) {
+    if (g.key == key && g.steps == steps) {
       *out = &g;
       return KW_OK;
     }
@@ -1367,10 +1380,12 @@ static int step_graph(kw_plan* p, int t, kw_plan::StepGraph** out) {
   const long long l0 = p->launches;
   CK(cudaStreamBeginCapture(p->cap_stream, cudaStreamCaptureModeRelaxed));
   p->capturing = true;
-  int rc = enqueue_step(p, t, false, p->cap_stream);
+  p->cap_t0 = t;
+  int rc = KW_OK;
+  for (int i = 0; i < steps && !rc; ++i) rc = enqueue_step(p, t + i, false, p->cap_stream);
   p->capturing = false;
   if (!rc) {
-    k_step_tick<<<1, 1, 0, p->cap_stream>>>(p->d_tstep);
+    k_step_tick<<<1, 1, 0, p->cap_stream>>>(p->d_tstep, steps);
     if (cudaGetLastError() != cudaSuccess) rc = fail(KW_ERR_CUDA, "step counter launch failed during capture");
   }
   cudaGraph_t graph = nullptr;
@@ -1388,7 +1403,7 @@ static int step_graph(kw_plan* p, int t, kw_plan::StepGraph** out) {
     cudaGraphDestroy(graph);
     return fail(KW_ERR_CUDA, "step graph instantiation: %s", cudaGetErrorString(ei));
   }
-  p->graphs.push_back(kw_plan::StepGraph{key, graph, exec, nl});
+  p->graphs.push_back(kw_plan::StepGraph{steps, key, graph, exec, nl});
   *out = &p->graphs.back();
   return KW_OK;
 }
@@ -1403,16 +1418,36 @@ static int step_counter_to(kw_plan* p, int t, cudaStream_t st) {
   return KW_OK;
 }
 
-static int run_step(kw_plan* p, int t, int end, cudaStream_t st) {
+static int run_step(kw_plan* p, int t, int end, cudaStream_t st, int steps = 1) {
   if (step_eager(p, t, end)) return enqueue_step(p, t, t == end - 1, st);
   kw_plan::StepGraph* g = nullptr;
-  int rc = step_graph(p, t, &g);
+  int rc = step_graph(p, t, steps, &g);
   if (!rc) rc = step_counter_to(p, t, st);
   if (rc) return rc;
   CK(cudaGraphLaunch(g->exec, st));
-  p->tstep_val = t + 1;
+  p->tstep_val = t + steps;
   p->launches += g->nlaunch;
   return KW_OK;
+}
+
+// Steps from t on that one graph launch may advance: kGraphSteps when that many
+// have the same key, none runs as plain launches and none but the last is
+// followed by a checkpoint, else 1.  The longer graph is captured only for runs
+// that use it at least four times.
+// (Between graphs the GPU idles for some microseconds; 604 steps of 128^2 took
+// 25.0 ms with a graph per step and plain edges, 22.3 with both changed.)
+constexpr int kGraphSteps = 8;
+static int graph_steps(kw_plan* p, int t, int end, int eend) {
+  if (step_eager(p, t, eend)) return 1;
+  const int key = step_key(p, t);
+  bool have = false;
+  for (const auto& g : p->graphs) have |= g.key == key && g.steps == kGraphSteps;
+  const int need = have ? kGraphSteps : 4 * kGraphSteps;
+  if (t + need > end) return 1;
+  if (p->ckpt_K > 0 && (t + p->ckpt_K - 1) / p->ckpt_K * p->ckpt_K < t + kGraphSteps - 1) return 1;
+  for (int i = 1; i < need; ++i)
+    if (step_eager(p, t + i, eend) || step_key(p, t + i) != key) return 1;
+  return kGraphSteps;
 }
 
 // plain_last == false (autotuning only): the last step is a graph step too and
@@ -1440,8 +1475,10 @@ static int plan_run(kw_plan* p, int nsteps, cudaStream_t st, bool plain_last) {
   const int end = std::min(p->g.Nt, p->t + nsteps);
   const int eend = plain_last ? end : end + 1;
   for (int t = p->t; t < end; ++t) {
-    int rc = run_step(p, t, eend, st);
+    const int steps = graph_steps(p, t, end, eend);
+    int rc = run_step(p, t, eend, st, steps);
     if (rc) return rc;
+    t += steps - 1;
     p->t = t + 1;
     if (p->ckpt_K > 0 && t % p->ckpt_K == 0) {
       const int s = t / p->ckpt_K;
@@ -1788,8 +1825,8 @@ int32_t kw_batch_create(kw_plan* const* plans, int32_t n, kw_batch** out) {
   // step graphs of batch members become child graphs: capture them with plain
   // stream-order edges between their kernels
   for (kw_plan* p : b->plans)
-    if (p->pdl) {
-      p->pdl = false;
+    if (p->pdl || p->mr_pdl) {
+      p->pdl = p->mr_pdl = false;
       drop_graphs(p);
     }
   *out = b;
@@ -1935,6 +1972,7 @@ static int batch_graph(kw_batch* b, const std::vector<int>& keys, kw_batch::Grap
     p->rec_nsm = std::max(1, p->nsm / (int)n);
     p->gated_src = mr && (keys[i] & kSrcKeyBits);
     p->capturing = true;
+    p->cap_t0 = p->t;
     rc = enqueue_step(p, p->t, false, nullptr);
     p->rec_list = nullptr;
     p->gated_src = false;
@@ -2039,7 +2077,7 @@ static int batch_graph(kw_batch* b, const std::vector<int>& keys, kw_batch::Grap
   std::vector<kw_plan::StepGraph*> sg(n, nullptr);
   for (size_t i = 0; i < n; ++i)
     if (keys[i] >= 0 && !G.grouped[i]) {
-      if ((rc = step_graph(b->plans[i], b->plans[i]->t, &sg[i]))) return rc;
+      if ((rc = step_graph(b->plans[i], b->plans[i]->t, 1, &sg[i]))) return rc;
       G.nl[i] = sg[i]->nlaunch;
     }
   if (!b->cap) CK(cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking));
@@ -2156,7 +2194,7 @@ static int batch_step_streams(kw_batch* b, const std::vector<int>& keys, cudaStr
   std::vector<kw_plan::StepGraph*> sg(n, nullptr);
   int rc;
   for (size_t i = 0; i < n; ++i)
-    if (keys[i] >= 0 && (rc = step_graph(b->plans[i], b->plans[i]->t, &sg[i]))) return rc;
+    if (keys[i] >= 0 && (rc = step_graph(b->plans[i], b->plans[i]->t, 1, &sg[i]))) return rc;
   CK(cudaEventRecord(b->fork_ev, st));
   for (size_t s = 0; s < ns; ++s) CK(cudaStreamWaitEvent(b->side[s], b->fork_ev, 0));
   for (size_t i = 0; i < n; ++i) {
