@@ -6,7 +6,7 @@
 #define KW_MR_AXIS_DECL(name)                                                                                    \
   cudaError_t kw_mr_axis_attr_##name(int smem);                                                                  \
   cudaError_t kw_mr_axis_go_##name(dim3 grid, int threads, size_t smem, cudaStream_t st, const MrAxisParams* W,  \
-                                   const MrAxisParams* Ps, const int2* map);
+                                   const MrAxisParams* Ps, const int2* map, bool pdl);
 KW_MR_AXIS_DECL(fwd)
 KW_MR_AXIS_DECL(inv)
 KW_MR_AXIS_DECL(grad)
@@ -98,22 +98,22 @@ cudaError_t kw_mr_axis_plan(const AxisParams& A, const KwMrLen& L, const float2*
 }
 
 static cudaError_t axis_go(int kind, dim3 grid, int threads, size_t smem, cudaStream_t st, const MrAxisParams* W,
-                           const MrAxisParams* Ps, const int2* map) {
+                           const MrAxisParams* Ps, const int2* map, bool pdl) {
   switch (kind) {
-    case MK_FWD: return kw_mr_axis_go_fwd(grid, threads, smem, st, W, Ps, map);
-    case MK_INV: return kw_mr_axis_go_inv(grid, threads, smem, st, W, Ps, map);
-    case MK_GRAD: return kw_mr_axis_go_grad(grid, threads, smem, st, W, Ps, map);
-    case MK_DIV: return kw_mr_axis_go_div(grid, threads, smem, st, W, Ps, map);
-    case MK_NAB: return kw_mr_axis_go_nab(grid, threads, smem, st, W, Ps, map);
-    default: return kw_mr_axis_go_gen(grid, threads, smem, st, W, Ps, map);
+    case MK_FWD: return kw_mr_axis_go_fwd(grid, threads, smem, st, W, Ps, map, pdl);
+    case MK_INV: return kw_mr_axis_go_inv(grid, threads, smem, st, W, Ps, map, pdl);
+    case MK_GRAD: return kw_mr_axis_go_grad(grid, threads, smem, st, W, Ps, map, pdl);
+    case MK_DIV: return kw_mr_axis_go_div(grid, threads, smem, st, W, Ps, map, pdl);
+    case MK_NAB: return kw_mr_axis_go_nab(grid, threads, smem, st, W, Ps, map, pdl);
+    default: return kw_mr_axis_go_gen(grid, threads, smem, st, W, Ps, map, pdl);
   }
 }
 
 cudaError_t kw_mr_axis_launch(const KwMrAxisLaunch& X, cudaStream_t st) {
-  return axis_go(X.kind, dim3(X.gx, X.gy), X.threads, X.smem, st, &X.W, nullptr, nullptr);
+  return axis_go(X.kind, dim3(X.gx, X.gy), X.threads, X.smem, st, &X.W, nullptr, nullptr, false);
 }
 
 cudaError_t kw_mr_axis_group_launch(int kind, int blocks, int threads, size_t smem, cudaStream_t st,
-                                    const MrAxisParams* Ps, const int2* map) {
-  return axis_go(kind, dim3(blocks), threads, smem, st, nullptr, Ps, map);
+                                    const MrAxisParams* Ps, const int2* map, bool pdl) {
+  return axis_go(kind, dim3(blocks), threads, smem, st, nullptr, Ps, map, pdl);
 }

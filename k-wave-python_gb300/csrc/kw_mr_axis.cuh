@@ -476,6 +476,7 @@ __global__ void __launch_bounds__(256, (KIND == MK_GRAD || KIND == MK_GEN) ? 2 :
   const int* src = reinterpret_cast<const int*>(Ps + me.x);
   for (int w = threadIdx.x; w < (int)(sizeof(MrAxisParams) / 4); w += blockDim.x) reinterpret_cast<int*>(&sp)[w] = src[w];
   __syncthreads();
+  kwtma::grid_dep_wait();
   if (sp.gate && *sp.gate >= sp.gate_end) return;
   const int item = me.y / sp.gx;
   mr_axis_body<KIND>(sp, me.y - item * sp.gx, item);
@@ -491,17 +492,14 @@ static cudaError_t kw_mr_axis_attr_kind(int smem) {
 // One plan's pass, or (Ps set) the grouped pass over `grid.x` blocks.
 template <int KIND>
 static cudaError_t kw_mr_axis_go(dim3 grid, int threads, size_t smem, cudaStream_t st, const MrAxisParams* W,
-                                 const MrAxisParams* Ps, const int2* map) {
-  if (Ps)
-    k_mr_axis_group<KIND><<<grid, threads, smem, st>>>(Ps, map);
-  else
-    return kwtma::launch_k(k_mr_axis<KIND>, grid, dim3(threads), smem, st, W->pdl, *W);
-  return cudaGetLastError();
+                                 const MrAxisParams* Ps, const int2* map, bool pdl) {
+  if (Ps) return kwtma::launch_k(k_mr_axis_group<KIND>, grid, dim3(threads), smem, st, pdl, Ps, map);
+  return kwtma::launch_k(k_mr_axis<KIND>, grid, dim3(threads), smem, st, W->pdl != 0, *W);
 }
 
 #define KW_MR_AXIS_DEFINE(name, KIND)                                                                              \
   cudaError_t kw_mr_axis_attr_##name(int smem) { return kw_mr_axis_attr_kind<KIND>(smem); }                        \
   cudaError_t kw_mr_axis_go_##name(dim3 grid, int threads, size_t smem, cudaStream_t st, const MrAxisParams* W,    \
-                                   const MrAxisParams* Ps, const int2* map) {                                      \
-    return kw_mr_axis_go<KIND>(grid, threads, smem, st, W, Ps, map);                                               \
+                                   const MrAxisParams* Ps, const int2* map, bool pdl) {                            \
+    return kw_mr_axis_go<KIND>(grid, threads, smem, st, W, Ps, map, pdl);                                          \
   }

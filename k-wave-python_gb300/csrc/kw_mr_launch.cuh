@@ -25,6 +25,6 @@ void kw_mr_rows_plan(int stage, int nsm, KwMrRowsLaunch& X);
 cudaError_t kw_mr_rows_launch(const KwMrRowsLaunch& X, cudaStream_t st);
 // Grouped: Ps[m] the members' parameters, map[i] = (member, its block) of block i.
 cudaError_t kw_mr_axis_group_launch(int kind, int blocks, int threads, size_t smem, cudaStream_t st,
-                                    const MrAxisParams* Ps, const int2* map);
+                                    const MrAxisParams* Ps, const int2* map, bool pdl);
 cudaError_t kw_mr_rows_group_launch(int stage, int dim, int blocks, int threads, size_t smem, cudaStream_t st,
-                                    const MrRowsParams* Ps, const int2* map);
+                                    const MrRowsParams* Ps, const int2* map, bool pdl);

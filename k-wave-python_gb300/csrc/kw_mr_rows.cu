@@ -5,7 +5,7 @@
 
 #define KW_MR_ROWS_DECL(i)                                                                                        \
   cudaError_t kw_mr_rows_go_##i(int stage, int odd, int dim, int blocks, int threads, size_t smem, cudaStream_t st, \
-                                const MrRowsParams* W, const MrRowsParams* Ps, const int2* map);
+                                const MrRowsParams* W, const MrRowsParams* Ps, const int2* map, bool pdl);
 KW_MR_ROWS_DECL(1)
 KW_MR_ROWS_DECL(2)
 KW_MR_ROWS_DECL(3)
@@ -54,19 +54,19 @@ void kw_mr_rows_plan(int stage, int nsm, KwMrRowsLaunch& X) {
 }
 
 static cudaError_t rows_go(int stage, int odd, int dim, int blocks, int threads, size_t smem, cudaStream_t st,
-                           const MrRowsParams* W, const MrRowsParams* Ps, const int2* map) {
-  if (stage == ST_U) return kw_mr_rows_go_1(stage, odd, dim, blocks, threads, smem, st, W, Ps, map);
-  if (stage == ST_RHO) return kw_mr_rows_go_2(stage, odd, dim, blocks, threads, smem, st, W, Ps, map);
-  if (stage == ST_EOS || stage == ST_SRC) return kw_mr_rows_go_3(stage, odd, dim, blocks, threads, smem, st, W, Ps, map);
-  if (stage >= ST_ADJ_A) return kw_mr_rows_go_4(stage, odd, dim, blocks, threads, smem, st, W, Ps, map);
-  return kw_mr_rows_go_5(stage, odd, dim, blocks, threads, smem, st, W, Ps, map);
+                           const MrRowsParams* W, const MrRowsParams* Ps, const int2* map, bool pdl) {
+  if (stage == ST_U) return kw_mr_rows_go_1(stage, odd, dim, blocks, threads, smem, st, W, Ps, map, pdl);
+  if (stage == ST_RHO) return kw_mr_rows_go_2(stage, odd, dim, blocks, threads, smem, st, W, Ps, map, pdl);
+  if (stage == ST_EOS || stage == ST_SRC) return kw_mr_rows_go_3(stage, odd, dim, blocks, threads, smem, st, W, Ps, map, pdl);
+  if (stage >= ST_ADJ_A) return kw_mr_rows_go_4(stage, odd, dim, blocks, threads, smem, st, W, Ps, map, pdl);
+  return kw_mr_rows_go_5(stage, odd, dim, blocks, threads, smem, st, W, Ps, map, pdl);
 }
 
 cudaError_t kw_mr_rows_launch(const KwMrRowsLaunch& X, cudaStream_t st) {
-  return rows_go(X.stage, X.odd, X.dim, X.blocks, X.threads, X.smem, st, &X.W, nullptr, nullptr);
+  return rows_go(X.stage, X.odd, X.dim, X.blocks, X.threads, X.smem, st, &X.W, nullptr, nullptr, false);
 }
 
 cudaError_t kw_mr_rows_group_launch(int stage, int dim, int blocks, int threads, size_t smem, cudaStream_t st,
-                                    const MrRowsParams* Ps, const int2* map) {
-  return rows_go(stage, 0, dim, blocks, threads, smem, st, nullptr, Ps, map);
+                                    const MrRowsParams* Ps, const int2* map, bool pdl) {
+  return rows_go(stage, 0, dim, blocks, threads, smem, st, nullptr, Ps, map, pdl);
 }

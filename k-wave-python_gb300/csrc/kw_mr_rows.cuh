@@ -763,7 +763,7 @@ __global__ void __launch_bounds__(KW_MR_THREADS, kw_mr_blocks(STAGE))
 // One plan's stage, or (Ps set) the grouped stage over `blocks` blocks.
 template <int STAGE, int DIM>
 static cudaError_t kw_mr_rows_go(int odd, int blocks, int threads, size_t smem, cudaStream_t st, const MrRowsParams* W,
-                                 const MrRowsParams* Ps, const int2* map) {
+                                 const MrRowsParams* Ps, const int2* map, bool pdl) {
   // one constant, so that plans of several threads never lower it under one another
   if (smem > 40 * 1024) {
     if (smem > KW_MR_ROWS_SMEM) return cudaErrorInvalidValue;
@@ -781,13 +781,11 @@ static cudaError_t kw_mr_rows_go(int odd, int blocks, int threads, size_t smem, 
             cudaFuncSetAttribute(k_mr_rows_group<STAGE, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, KW_MR_ROWS_SMEM);
         if (e != cudaSuccess) return e;
       }
-      k_mr_rows_group<STAGE, DIM><<<blocks, threads, smem, st>>>(Ps, map);
+      return kwtma::launch_k(k_mr_rows_group<STAGE, DIM>, dim3(blocks), dim3(threads), smem, st, pdl, Ps, map);
     } else {
       return cudaErrorInvalidValue;
     }
-  } else if (odd)
-    return kwtma::launch_k(k_mr_rows<STAGE, true, DIM>, dim3(blocks), dim3(threads), smem, st, W->pdl, *W);
-  else
-    return kwtma::launch_k(k_mr_rows<STAGE, false, DIM>, dim3(blocks), dim3(threads), smem, st, W->pdl, *W);
-  return cudaGetLastError();
+  }
+  if (odd) return kwtma::launch_k(k_mr_rows<STAGE, true, DIM>, dim3(blocks), dim3(threads), smem, st, W->pdl != 0, *W);
+  return kwtma::launch_k(k_mr_rows<STAGE, false, DIM>, dim3(blocks), dim3(threads), smem, st, W->pdl != 0, *W);
 }

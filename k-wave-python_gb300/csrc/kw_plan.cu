@@ -1884,8 +1884,16 @@ static bool batch_keys(kw_batch* b, int m, const std::vector<int>& end, const st
 }
 
 // Launch k of the members is one grouped launch where their sequences agree;
-// otherwise the longest remaining sequence goes first.  `chains` independent
-// sets of members run beside each other.
+// otherwise the longest remaining sequence goes first.
+//
+// A batch's members are dealt to three chains of such launches that run beside
+// each other, so that one chain's launches fill the SMs that another's last wave
+// leaves (the last waves took a third of the passes with 600 to 700 blocks), and
+// launches within a chain are programmatic dependents.  500 steps of 32 grids of
+// 192 to 512 points a side: one chain 295 ms, two 256, three 254, eight 258, three
+// with dependents 253; of 4 grids of 384 to 640: 128, 114, 104, -, 100.
+constexpr size_t kBatchChains = 3;
+
 struct MrGroup {
   int kind;  // LaunchRec::kind 3 or 4
   int stage, dim, akind;
@@ -2048,13 +2056,28 @@ static int batch_graph(kw_batch* b, const std::vector<int>& keys, kw_batch::Grap
       q.blk = static_cast<int4*>(dblk);
       pend.push_back(q);
     }
-  std::vector<MrGroup> mrg;
+  // members on the mixed-radix kernels: largest first to the chain with the least work
+  std::vector<std::vector<MrGroup>> chains;
   {
-    std::vector<const std::vector<kw_plan::LaunchRec>*> ml;
+    std::vector<size_t> order;
     for (size_t i = 0; i < n; ++i)
-      if (G.grouped[i] == 2) ml.push_back(&lists[i]);
-    mr_groups(ml, mrg);
-    for (MrGroup& g : mrg) {
+      if (G.grouped[i] == 2) order.push_back(i);
+    std::sort(order.begin(), order.end(), [&](size_t i, size_t j) { return b->plans[i]->ntot > b->plans[j]->ntot; });
+    const size_t nc = std::min(kBatchChains, order.size());
+    std::vector<std::vector<const std::vector<kw_plan::LaunchRec>*>> ml(nc);
+    std::vector<long long> load(nc, 0);
+    for (size_t i : order) {
+      const size_t c = std::min_element(load.begin(), load.end()) - load.begin();
+      ml[c].push_back(&lists[i]);
+      load[c] += b->plans[i]->ntot;
+    }
+    chains.resize(nc);
+    for (size_t c = 0; c < nc; ++c) mr_groups(ml[c], chains[c]);
+    std::vector<MrGroup*> groups;
+    for (auto& c : chains)
+      for (MrGroup& g : c) groups.push_back(&g);
+    for (MrGroup* gp : groups) {
+      MrGroup& g = *gp;
       void* d = nullptr;
       if (g.kind == 3) {
         if ((rc = batch_upload(b, g.rp.data(), g.rp.size() * sizeof(MrRowsParams), &d))) return rc;
@@ -2095,20 +2118,43 @@ static int batch_graph(kw_batch* b, const std::vector<int>& keys, kw_batch::Grap
                   : kw_axis_group_launch_0(q.total, q.smem, b->cap, aq, q.blk, q.m);
     if (elaunch == cudaSuccess) elaunch = e;
   }
-  for (const MrGroup& g : mrg) {
-    const cudaError_t e = g.kind == 3 ? kw_mr_rows_group_launch(g.stage, g.dim, g.blocks, g.threads, g.smem, b->cap, g.d_rp, g.d_map)
-                                      : kw_mr_axis_group_launch(g.akind, g.blocks, g.threads, g.smem, b->cap, g.d_ap, g.d_map);
+  auto keep = [&](cudaError_t e) {
     if (elaunch == cudaSuccess) elaunch = e;
+  };
+  std::vector<cudaStream_t> side(chains.size(), b->cap);
+  std::vector<cudaEvent_t> marks(chains.size(), nullptr);  // the fork, then the ends of the side chains
+  for (auto& e : marks) keep(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  if (chains.size() > 1) keep(cudaEventRecord(marks[0], b->cap));
+  for (size_t c = 0; c < chains.size(); ++c) {
+    if (c) {
+      keep(cudaStreamCreateWithFlags(&side[c], cudaStreamNonBlocking));
+      keep(cudaStreamWaitEvent(side[c], marks[0], 0));
+    }
+    for (const MrGroup& g : chains[c]) {
+      const bool pdl = &g != &chains[c][0];
+      keep(g.kind == 3
+               ? kw_mr_rows_group_launch(g.stage, g.dim, g.blocks, g.threads, g.smem, side[c], g.d_rp, g.d_map, pdl)
+               : kw_mr_axis_group_launch(g.akind, g.blocks, g.threads, g.smem, side[c], g.d_ap, g.d_map, pdl));
+    }
+  }
+  for (size_t c = 1; c < chains.size(); ++c) {
+    keep(cudaEventRecord(marks[c], side[c]));
+    keep(cudaStreamWaitEvent(b->cap, marks[c], 0));
   }
   if (dticks) k_step_tick_group<<<((int)ticks.size() + 127) / 128, 128, 0, b->cap>>>(dticks, (int)ticks.size());
   const cudaError_t el = elaunch != cudaSuccess ? elaunch : cudaGetLastError();
   cudaGraph_t graph = nullptr;
   const cudaError_t ec = cudaStreamEndCapture(b->cap, &graph);
+  for (size_t c = 1; c < side.size(); ++c)
+    if (side[c] != b->cap) cudaStreamDestroy(side[c]);
+  for (cudaEvent_t e : marks)
+    if (e) cudaEventDestroy(e);
   if (el != cudaSuccess || ec != cudaSuccess) {
     if (graph) cudaGraphDestroy(graph);
     return fail(KW_ERR_CUDA, "batch capture: %s", cudaGetErrorString(el != cudaSuccess ? el : ec));
   }
-  G.nlaunch = (long long)(pend.size() + mrg.size()) + (dticks ? 1 : 0);
+  G.nlaunch = (long long)pend.size() + (dticks ? 1 : 0);
+  for (const auto& c : chains) G.nlaunch += (long long)c.size();
   for (size_t i = 0; i < n; ++i) {
     if (!sg[i]) continue;
     cudaGraphNode_t node;
