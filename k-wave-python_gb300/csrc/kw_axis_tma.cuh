@@ -346,6 +346,7 @@ __global__ void __launch_bounds__(T * P + 32, MINB)
           for (int j = 0; j < E; ++j) v[j] = st[(t + P * j) * T + cc];
         }
         if constexpr (!TSTORE) {
+          kwtma::fence_proxy_async_smem();  // this lane's reads before the copy that refills the slot
           __syncwarp();
           if (lane == 0) kwtma::mbar_arrive(&empty[s]);
         }

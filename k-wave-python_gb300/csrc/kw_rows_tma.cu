@@ -191,7 +191,11 @@ __global__ void __launch_bounds__(160, row_ctas(STAGE)) k_rows_tma(const __grid_
       }
       return reinterpret_cast<const float2*>(slots + (size_t)s * slot_bytes);
     };
+    // (the fence: this lane's reads of the slot are done before the copy that refills
+    // it, which the async proxy writes; reads still queued in the shared-memory pipe
+    // at the arrival saw the next copy's data)
     auto release = [&](uint32_t i) {
+      kwtma::fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) kwtma::mbar_arrive(&empty[i % NST]);
     };
