@@ -261,7 +261,7 @@ int kw_device_error_take();
 // Device address of that word on the current device (nullptr on failure).
 int* kw_device_error_ptr();
 // Velocity and power-law density stages fed by bulk copies (kw_rows_tma.cu),
-// power-of-two row lengths; stage is ST_U or ST_RHO_PL.
+// power-of-two row lengths; stage is ST_U, ST_RHO (linear, no power law), ST_RHO_PL or ST_EOS.
 cudaError_t kw_rows_tma_attr(int m, int Hp, int ex_stride);
 cudaError_t kw_rows_tma_launch(int m, int stage, int nsm, cudaStream_t st, const RowsParams& Q, int* err, int pdl);
 __global__ void k_series_gather(const float* __restrict__ rec, int nrec, int nslots, int npts, int ncorner,

@@ -109,7 +109,7 @@ struct kw_plan {
   // persistent TMA axis passes
   void* tma = nullptr;
   bool tma_axis[3] = {false, false, false};
-  bool rows_tma = false;  // velocity / power-law density stages through kw_rows_tma
+  bool rows_tma = false;  // velocity, density and equation-of-state stages through kw_rows_tma
   // kw_plan_derive_medium request
   int derive_what = 0;
   std::vector<float> halpha;
@@ -1056,6 +1056,9 @@ static int launch_rows(kw_plan* p, int stage, int init, int t, int write_p, cuda
     }
     else if (stage == ST_RHO && dsm && !extra && p->rows_tma)
       CK(kw_rows_tma_launch(p->Mfft, ST_RHO_PL, p->nsm, st, P, kw_device_error_ptr(), pdl_ok(p)));
+    // (the nonlinear factor needs every density before the first: register kernel)
+    else if (stage == ST_RHO && P.absorb != 1 && !P.nonlin && !extra && p->rows_tma)
+      CK(kw_rows_tma_launch(p->Mfft, ST_RHO, p->nsm, st, P, kw_device_error_ptr(), pdl_ok(p)));
     else if (stage == ST_EOS && p->rows_tma)
       CK(kw_rows_tma_launch(p->Mfft, ST_EOS, p->nsm, st, P, kw_device_error_ptr(), pdl_ok(p)));
     else {

@@ -16,6 +16,12 @@
 //             S_a, rho_a; split-density update with power-law absorption
 //             (kspace_solver.py:709-717, :498, :524), as the register
 //             kernel's ST_RHO_PL
+//   ST_RHO    the density stage of linear media without power-law absorption:
+//             rho0 (if a grid), per component a: S_a, rho_a, then (Stokes) tau and
+//             rho0, c0 (if grids); equation of state (kspace_solver.py:709-723), as
+//             the register kernel's ST_RHO.  Bound by DRAM: 128 x 256 x 256 points
+//             of water took 156 us on the register kernel, 87 here (about 370 MB);
+//             64 x 64 x 1024 270 and 167
 //   ST_EOS    the two fractional-Laplacian spectra, sum rho, tau, eta, rho0,
 //             B/A, c0 (those that are grids); equation of state with
 //             absorption and dispersion (kspace_solver.py:719-723)
@@ -32,7 +38,7 @@ constexpr uint64_t kRowWaitNs = 2000000000ull;
 // Ring depth and resident CTAs per SM per stage: the density stage keeps its
 // density-sum slots in shared memory and needs more registers (2 CTAs, 4
 // slots); the velocity and EOS stages run 3 CTAs of 3 slots.
-__host__ __device__ constexpr int row_nst(int stage) { return stage == ST_RHO_PL ? 2 : 3; }
+__host__ __device__ constexpr int row_nst(int stage) { return stage == ST_RHO_PL || stage == ST_RHO ? 2 : 3; }
 __host__ __device__ constexpr int row_ctas(int stage) { return 3; }
 
 __device__ __forceinline__ bool consumers_any_rows(bool pred, int n) {
@@ -70,6 +76,15 @@ __device__ __forceinline__ const void* row_load(const RowsParams& Q, int idx, bo
       case 6: return Q.nonlin ? Q.bona : nullptr;
       default: return Q.c0;
     }
+  } else if constexpr (STAGE == ST_RHO) {
+    const int tail = idx - 1 - 2 * D;
+    spec = idx >= 1 && tail < 0 && (idx & 1);
+    if (idx == 0) return Q.rho0;
+    if (tail == 0) return Q.absorb == 2 ? Q.tau : nullptr;
+    if (tail == 1) return Q.absorb == 2 ? Q.rho0 : nullptr;
+    if (tail == 2) return Q.c0;
+    const int a = (idx - 1) >> 1;
+    return spec ? (const void*)Q.S[a] : (const void*)Q.rho[a];
   } else {
     if (idx == 0) {
       spec = false;
@@ -91,7 +106,7 @@ __device__ __forceinline__ const void* row_load(const RowsParams& Q, int idx, bo
 
 template <int STAGE>
 __device__ __forceinline__ int row_nloads(const RowsParams& Q) {
-  return STAGE == ST_U ? 3 * Q.ndim : STAGE == ST_EOS ? 8 : 3 + 2 * Q.ndim;
+  return STAGE == ST_U ? 3 * Q.ndim : STAGE == ST_EOS ? 8 : STAGE == ST_RHO ? 4 + 2 * Q.ndim : 3 + 2 * Q.ndim;
 }
 
 }  // namespace
@@ -109,10 +124,10 @@ __global__ void __launch_bounds__(160, row_ctas(STAGE)) k_rows_tma(const __grid_
   float2* tw = reinterpret_cast<float2*>(slots + (size_t)NST * slot_bytes);
   float2* twp = tw + M;
   float2* ex = twp + (M + 1);
-  // ST_RHO_PL: the new density sum accumulates in this thread's slots
+  // density stages: the new density sum accumulates in this thread's slots
   // (rsm[j * 128 + thread]) instead of registers
   float2* rsm = ex + R * Q.ex_stride;
-  constexpr int NRS = STAGE == ST_RHO_PL ? 128 * E : 0;
+  constexpr int NRS = STAGE == ST_RHO_PL || STAGE == ST_RHO ? 128 * E : 0;
   // the stage's PML profile along the last axis (2 M reals), read per element
   float* pmlz = reinterpret_cast<float*>(rsm + NRS);
   uint64_t* full = reinterpret_cast<uint64_t*>((reinterpret_cast<uintptr_t>(pmlz + 2 * M) + 7) & ~uintptr_t(7));
@@ -130,7 +145,7 @@ __global__ void __launch_bounds__(160, row_ctas(STAGE)) k_rows_tma(const __grid_
   }
   for (int i = tid; i < M; i += blockDim.x) tw[i] = Q.tw[i];
   for (int i = tid; i <= M; i += blockDim.x) twp[i] = Q.twpost[i];
-  if constexpr (STAGE == ST_U || STAGE == ST_RHO_PL) {
+  if constexpr (STAGE == ST_U || STAGE == ST_RHO_PL || STAGE == ST_RHO) {
     const float* src = STAGE == ST_U ? Q.pmlsg[D - 1] : Q.pml[D - 1];
     for (int i = tid; i < 2 * M; i += blockDim.x) pmlz[i] = src[i];
   }
@@ -327,6 +342,88 @@ __global__ void __launch_bounds__(160, row_ctas(STAGE)) k_rows_tma(const __grid_
         if (sf) release(it++);
         c.record(v, Q.rec[0]);
         c.r2c(v, Q.S[3]);
+      } else if constexpr (STAGE == ST_RHO) {
+        float2 w[E], div[E];  // dt rho0; divergence (Stokes absorption)
+        const float2* sf = nullptr;
+        if (Q.rho0) {
+          sf = wait_item(it);
+          if (!sf) break;
+        }
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+          const float2 r0 = sf ? sf[row * M + t + P * j] : make_float2(Q.rho0_s, Q.rho0_s);
+          w[j] = make_float2(__fmul_rn(Q.dt, r0.x), __fmul_rn(Q.dt, r0.y));
+          div[j] = make_float2(0.f, 0.f);
+        }
+        if (sf) release(it++);
+        for (int a = 0; a < D; ++a) {
+          const float2* ss = wait_item(it);
+          if (!ss) break;
+          c.c2r_row(ss + row * Hp, v);
+          release(it++);
+          const float2* sr = wait_item(it);
+          if (!sr) break;
+          const float2* rrow = sr + row * M;
+#pragma unroll
+          for (int j = 0; j < E; ++j) {
+            const int n = t + P * j;
+            const float2 du = v[j];
+            div[j] = make_float2(__fadd_rn(div[j].x, du.x), __fadd_rn(div[j].y, du.y));
+            if (!c.ok) continue;
+            const float2 pm = c.pml2(a == D - 1 ? pmlz : Q.pml[a], a, n);
+            const float2 ro = rrow[n];
+            v[j] = make_float2(__fmul_rn(pm.x, __fsub_rn(__fmul_rn(pm.x, ro.x), __fmul_rn(w[j].x, du.x))),
+                               __fmul_rn(pm.y, __fsub_rn(__fmul_rn(pm.y, ro.y), __fmul_rn(w[j].y, du.y))));
+          }
+          release(it++);
+          c.source(Q.src[a], v);
+#pragma unroll
+          for (int j = 0; j < E; ++j) {
+            if (c.ok) st2(Q.rho[a], c.rbase + t + P * j, v[j]);
+            float2* rp = rsm + j * CT + tid;
+            const float2 r = (a == 0) ? v[j] : *rp;
+            *rp = (a == 0) ? r : make_float2(__fadd_rn(r.x, v[j].x), __fadd_rn(r.y, v[j].y));
+          }
+        }
+        if (aborted) break;
+        if (Q.absorb == 2) {
+          sf = nullptr;
+          if (Q.tau) {
+            sf = wait_item(it);
+            if (!sf) break;
+          }
+#pragma unroll
+          for (int j = 0; j < E; ++j) w[j] = sf ? sf[row * M + t + P * j] : make_float2(Q.tau_s, Q.tau_s);
+          if (sf) release(it++);
+          sf = nullptr;
+          if (Q.rho0) {
+            sf = wait_item(it);
+            if (!sf) break;
+          }
+#pragma unroll
+          for (int j = 0; j < E; ++j) {
+            const float2 r0 = sf ? sf[row * M + t + P * j] : make_float2(Q.rho0_s, Q.rho0_s);
+            div[j] = make_float2(__fmul_rn(__fmul_rn(w[j].x, r0.x), div[j].x), __fmul_rn(__fmul_rn(w[j].y, r0.y), div[j].y));
+          }
+          if (sf) release(it++);
+        }
+        sf = nullptr;
+        if (Q.c0) {
+          sf = wait_item(it);
+          if (!sf) break;
+        }
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+          const float2 cc = sf ? sf[row * M + t + P * j] : make_float2(Q.c0_s, Q.c0_s);
+          float2 acc = rsm[j * CT + tid];
+          if (Q.absorb == 2) acc = make_float2(__fadd_rn(acc.x, div[j].x), __fadd_rn(acc.y, div[j].y));
+          v[j] = c.ok ? make_float2(__fmul_rn(__fmul_rn(cc.x, cc.x), acc.x), __fmul_rn(__fmul_rn(cc.y, cc.y), acc.y))
+                      : make_float2(0.f, 0.f);
+          if (c.ok && Q.write_p) st2(Q.p, c.rbase + t + P * j, v[j]);
+        }
+        if (sf) release(it++);
+        c.record(v, Q.rec[0]);
+        c.r2c(v, Q.S[3]);
       } else {
         // w = dt rho0 (2 sum rho + rho0) / rho0 per pair (nonlinear factor from
         // the previous step's density sum), rho0 kept for rho0 * div
@@ -425,7 +522,7 @@ static size_t rows_tma_smem(int stage, int M, int E, int P, int Hp, int ex_strid
   const int R = 128 / P;
   const size_t spec_row = (size_t)Hp * 8, fld_row = (size_t)M * 8;
   const size_t slot = ((R * (spec_row > fld_row ? spec_row : fld_row)) + 127) & ~(size_t)127;
-  const size_t nrs = stage == ST_RHO_PL ? (size_t)128 * E : 0;
+  const size_t nrs = stage == ST_RHO_PL || stage == ST_RHO ? (size_t)128 * E : 0;
   const int nst = row_nst(stage);
   return nst * slot + sizeof(float2) * (2 * (size_t)M + 1 + (size_t)R * ex_stride + nrs) + sizeof(float) * 2 * M + 8 +
          2 * nst * 8 + 16;
@@ -469,11 +566,13 @@ static cudaError_t rows_tma_launch(int m, int nsm, cudaStream_t st, const RowsPa
 cudaError_t kw_rows_tma_attr(int m, int Hp, int ex_stride) {
   cudaError_t e = rows_tma_attr<ST_U>(m, Hp, ex_stride);
   if (e == cudaSuccess) e = rows_tma_attr<ST_RHO_PL>(m, Hp, ex_stride);
+  if (e == cudaSuccess) e = rows_tma_attr<ST_RHO>(m, Hp, ex_stride);
   return e == cudaSuccess ? rows_tma_attr<ST_EOS>(m, Hp, ex_stride) : e;
 }
 
 cudaError_t kw_rows_tma_launch(int m, int stage, int nsm, cudaStream_t st, const RowsParams& Q, int* err, int pdl) {
   if (stage == ST_U) return rows_tma_launch<ST_U>(m, nsm, st, Q, err, pdl);
+  if (stage == ST_RHO) return rows_tma_launch<ST_RHO>(m, nsm, st, Q, err, pdl);
   if (stage == ST_RHO_PL) return rows_tma_launch<ST_RHO_PL>(m, nsm, st, Q, err, pdl);
   if (stage == ST_EOS) return rows_tma_launch<ST_EOS>(m, nsm, st, Q, err, pdl);
   return cudaErrorInvalidValue;
