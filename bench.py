@@ -658,7 +658,7 @@ def run_transmit(args):
         "ms_per_step": ms / K_steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic (seeded speckle media, discs, steering angles and grid sizes of the named ranges)",
         "config": {"workload": TRANSMIT_WORKLOAD, "instances": ninst, "cells_per_step": cells, "nt": nt,
-                   "batch": "grouped launches" if args.grouped else "members as parallel graph branches",
+                   "batch": "grouped launches" if args.grouped else "members in chains of grouped launches",
                    "autotune": bool(args.autotune), "tuned": tuned, "radix_autotune": bool(args.radix),
                    "radix_order": radix_order, "setup_seconds": t_setup,
                    "l2": f"inputs larger than L2 ({cells * 4 * 12 / 1e9:.1f} GB of state, medium and spectra)"},

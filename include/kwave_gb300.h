@@ -160,8 +160,8 @@ int32_t kw_plan_finalize(kw_plan* plan);
  * call, the t = 0 initial-condition step and every step while timing is on are
  * plain launches.  Use one stream per plan. */
 int32_t kw_plan_run(kw_plan* plan, int32_t nsteps, void* stream);
-/* Autotuner of the run-time-length FFT kernels (the lengths that are not
- * powers of two): times `nsteps` graph steps after the t = 0 step (at least
+/* Autotuner of the run-time-length FFT kernels (lengths with a prime factor
+ * above 7, and plans of KW_DESC_GENERIC_FFT): times `nsteps` graph steps after the t = 0 step (at least
  * 2, at most Nt - 1) for each candidate launch geometry -- tile columns T in
  * {2, 4, 8, 16} of the axis passes, rows per block R in {R0/2, R0, 2 R0} of
  * the row stages -- keeps the fastest and rewinds the plan to t = 0
