@@ -79,6 +79,8 @@ bool kw_tma_encode(void* h, int axis, int b, void* base, int ncols, int n, long 
   return r == CUDA_SUCCESS;
 }
 
+bool kw_tma_plain_shape(int n, int* E, int* P) { return kw_tma_shape(n, KK_PLAIN, E, P); }
+
 bool kw_tma_supported(int n) {
   int E, P;
   return encode_fn() != nullptr && kw_reg_shape(n, &E, &P);

@@ -137,12 +137,12 @@ struct TabX {
 // into the spectrum).
 template <int OP>
 __device__ __forceinline__ float2 op_value(const AxisParams& A, const AxisJob& J, int x, const ColK& g,
-                                           const float* k0s, const TabX& f0s, float2 fcol, bool full) {
+                                           const float* k0s, const TabX& f0s, float2 fcol, bool full, float lo) {
   float2 op = make_float2(0.f, 0.f);
   if constexpr (OP == OP_GRAD || OP == OP_DIV) {
     const float2 f = (J.axis == 0) ? (OP == OP_GRAD ? f0s.grad[x] : f0s.div[x]) : fcol;
     if (!full) return f;
-    const float kp = kappa_of(A, kmag_of(k0s, A.ndim, x, g)) * A.scale;
+    const float kp = scaled(A, kappa_of(A, kmag_of(k0s, A.ndim, x, g)), lo);
     return make_float2(f.x * kp, f.y * kp);
   } else if constexpr (OP == OP_NAB1 || OP == OP_NAB2) {
     const float km = kmag_of(k0s, A.ndim, x, g);
@@ -156,36 +156,36 @@ __device__ __forceinline__ float2 op_value(const AxisParams& A, const AxisJob& J
   } else {
     op = (J.axis == 0) ? f0s.unstag[x] : fcol;
   }
-  return make_float2(op.x * A.scale, op.y * A.scale);
+  return make_float2(scaled(A, op.x, lo), scaled(A, op.y, lo));
 }
 
 // y[r] = conj(op * v[r]) over the thread's frequencies, for operator OP.
 template <int OP, int E, int P>
 __device__ __forceinline__ void apply_op(const AxisParams& A, const AxisJob& J, int t, const ColK& g, const float* k0s,
-                                         const TabX& f0s, float2 fcol, bool full, bool on, const float2 (&v)[E],
+                                         const TabX& f0s, float2 fcol, bool full, float lo, bool on, const float2 (&v)[E],
                                          float2 (&y)[E]) {
 #pragma unroll
   for (int m = 0; m < E / P; ++m)
 #pragma unroll
     for (int k2 = 0; k2 < P; ++k2) {
       const int r = m * P + k2;
-      const float2 op = op_value<OP>(A, J, t + P * m + E * k2, g, k0s, f0s, fcol, full);
+      const float2 op = op_value<OP>(A, J, t + P * m + E * k2, g, k0s, f0s, fcol, full, lo);
       y[r] = on ? cconj(kwreg::cmulf(op, v[r])) : make_float2(0.f, 0.f);
     }
 }
 
 template <int E, int P>
 __device__ __forceinline__ void apply_job(const AxisParams& A, const AxisJob& J, int t, const ColK& g, const float* k0s,
-                                          const TabX& f0s, float2 fcol, bool full, bool on, const float2 (&v)[E],
+                                          const TabX& f0s, float2 fcol, bool full, float lo, bool on, const float2 (&v)[E],
                                           float2 (&y)[E]) {
   switch (J.op) {
-    case OP_GRAD: apply_op<OP_GRAD, E, P>(A, J, t, g, k0s, f0s, fcol, full, on, v, y); break;
-    case OP_DIV: apply_op<OP_DIV, E, P>(A, J, t, g, k0s, f0s, fcol, full, on, v, y); break;
-    case OP_NAB1: apply_op<OP_NAB1, E, P>(A, J, t, g, k0s, f0s, fcol, full, on, v, y); break;
-    case OP_NAB2: apply_op<OP_NAB2, E, P>(A, J, t, g, k0s, f0s, fcol, full, on, v, y); break;
-    case OP_SKAPPA: apply_op<OP_SKAPPA, E, P>(A, J, t, g, k0s, f0s, fcol, full, on, v, y); break;
-    case OP_WIN: apply_op<OP_WIN, E, P>(A, J, t, g, k0s, f0s, fcol, full, on, v, y); break;
-    default: apply_op<OP_UNSTAG, E, P>(A, J, t, g, k0s, f0s, fcol, full, on, v, y); break;
+    case OP_GRAD: apply_op<OP_GRAD, E, P>(A, J, t, g, k0s, f0s, fcol, full, lo, on, v, y); break;
+    case OP_DIV: apply_op<OP_DIV, E, P>(A, J, t, g, k0s, f0s, fcol, full, lo, on, v, y); break;
+    case OP_NAB1: apply_op<OP_NAB1, E, P>(A, J, t, g, k0s, f0s, fcol, full, lo, on, v, y); break;
+    case OP_NAB2: apply_op<OP_NAB2, E, P>(A, J, t, g, k0s, f0s, fcol, full, lo, on, v, y); break;
+    case OP_SKAPPA: apply_op<OP_SKAPPA, E, P>(A, J, t, g, k0s, f0s, fcol, full, lo, on, v, y); break;
+    case OP_WIN: apply_op<OP_WIN, E, P>(A, J, t, g, k0s, f0s, fcol, full, lo, on, v, y); break;
+    default: apply_op<OP_UNSTAG, E, P>(A, J, t, g, k0s, f0s, fcol, full, lo, on, v, y); break;
   }
 }
 
@@ -397,11 +397,12 @@ __global__ void __launch_bounds__(T * P + 32, MINB)
         } else if constexpr (KIND == KK_GRAD) {
           kwreg::Reg<E, P>::fwd_t(v, t, exr, 1, tw, sync);
           // the D gradients share kappa(|k|) / N: fold it into the spectrum once
+          const float lo = col_scale_lo(A, g.a1, g.a2, g.valid);
 #pragma unroll
           for (int m = 0; m < E / P; ++m)
 #pragma unroll
             for (int k2 = 0; k2 < P; ++k2) {
-              const float kp = kappa_kk(A, kk_of(k0s, A.ndim, t + P * m + E * k2, g)) * A.scale;
+              const float kp = scaled(A, kappa_kk(A, kk_of(k0s, A.ndim, t + P * m + E * k2, g)), lo);
               v[m * P + k2] = make_float2(v[m * P + k2].x * kp, v[m * P + k2].y * kp);
             }
           // x derivative: its 1-D operator varies along x
@@ -435,11 +436,12 @@ __global__ void __launch_bounds__(T * P + 32, MINB)
           // item q is the velocity spectrum of axis q; its derivative replaces it
           kwreg::Reg<E, P>::fwd_t(v, t, exr, 1, tw, sync);
           if (q == 0) {
+            const float lo = col_scale_lo(A, g.a1, g.a2, g.valid);
 #pragma unroll
             for (int m = 0; m < E / P; ++m)
 #pragma unroll
               for (int k2 = 0; k2 < P; ++k2)
-                kc[m * P + k2] = kappa_kk(A, kk_of(k0s, A.ndim, t + P * m + E * k2, g)) * A.scale;
+                kc[m * P + k2] = scaled(A, kappa_kk(A, kk_of(k0s, A.ndim, t + P * m + E * k2, g)), lo);
           }
           const float2 fcol = col_factor_of(A, OP_DIV, q, g);
 #pragma unroll
@@ -461,17 +463,18 @@ __global__ void __launch_bounds__(T * P + 32, MINB)
 #pragma unroll
               for (int k2 = 0; k2 < P; ++k2) kc[m * P + k2] = log2f(kk_of(k0s, A.ndim, t + P * m + E * k2, g));
           }
-          const float hp = 0.5f * (q == 0 ? A.pow1 : A.pow2);
+          const float hp = 0.5f * (q == 0 ? A.pow1 : A.pow2), lo = col_scale_lo(A, g.a1, g.a2, g.valid);
 #pragma unroll
           for (int r = 0; r < E; ++r) {
             const float val = (kc[r] == -INFINITY) ? 0.f : exp2f(hp * kc[r]);
-            const float2 op = make_float2(val * A.scale, 0.f);
-            v[r] = on ? cconj(kwreg::cmulf(op, v[r])) : make_float2(0.f, 0.f);
+            const float a = scaled(A, val, lo);
+            v[r] = on ? make_float2(v[r].x * a, -(v[r].y * a)) : make_float2(0.f, 0.f);
           }
           store_rev(v, W.inp[q]);
         } else {
           // generic operator mode: forward FFT of this input, then every job reading it
           kwreg::Reg<E, P>::fwd_t(v, t, exr, 1, tw, sync);
+          const float lo = col_scale_lo(A, g.a1, g.a2, g.valid);
           const int in = W.inp[q];
           int nj = 0, jlast = 0;
           bool all_kappa = true;
@@ -485,7 +488,7 @@ __global__ void __launch_bounds__(T * P + 32, MINB)
             // one job: multiply in place
             const AxisJob J = A.jobs[jlast];
             const float2 fcol = col_factor(A, J, g);
-            apply_job<E, P>(A, J, t, g, k0s, f0s, fcol, true, on, v, v);
+            apply_job<E, P>(A, J, t, g, k0s, f0s, fcol, true, lo, on, v, v);
             rev_store<E, P>(v, t, exr, twr, sync, act, A.bufs[J.out], base, xs);
             continue;
           }
@@ -495,7 +498,7 @@ __global__ void __launch_bounds__(T * P + 32, MINB)
             for (int m = 0; m < E / P; ++m)
 #pragma unroll
               for (int k2 = 0; k2 < P; ++k2) {
-                const float kp = kappa_of(A, kmag_of(k0s, A.ndim, t + P * m + E * k2, g)) * A.scale;
+                const float kp = scaled(A, kappa_of(A, kmag_of(k0s, A.ndim, t + P * m + E * k2, g)), lo);
                 v[m * P + k2] = make_float2(v[m * P + k2].x * kp, v[m * P + k2].y * kp);
               }
           }
@@ -504,7 +507,7 @@ __global__ void __launch_bounds__(T * P + 32, MINB)
             if (J.in != in) continue;
             const float2 fcol = col_factor(A, J, g);
             float2 y[E];
-            apply_job<E, P>(A, J, t, g, k0s, f0s, fcol, !all_kappa, on, v, y);
+            apply_job<E, P>(A, J, t, g, k0s, f0s, fcol, !all_kappa, lo, on, v, y);
             rev_store<E, P>(y, t, exr, twr, sync, act, A.bufs[J.out], base, xs);
           }
         }

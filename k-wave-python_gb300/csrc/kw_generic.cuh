@@ -67,7 +67,8 @@ static __device__ __forceinline__ float2 axis_op(const AxisParams& P, const Axis
       v = P.us[J.axis][ai];
       break;
   }
-  return make_float2(v.x * P.scale, v.y * P.scale);
+  const float lo = col_scale_lo(P, a1, a2, true);
+  return make_float2(scaled(P, v.x, lo), scaled(P, v.y, lo));
 }
 
 // ---------------------------------------------------------------------------

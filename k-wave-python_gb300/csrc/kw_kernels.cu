@@ -19,7 +19,7 @@ __global__ void k_step_tick_group(int* const* __restrict__ tdev, int n) {
 // register-FFT variants for power-of-two lengths (kw_regfft.cuh)
 // ---------------------------------------------------------------------------
 // Spectral operator value at x-frequency index x of a column (register axis pass).
-__device__ __forceinline__ float2 col_op(const AxisParams& A, const AxisJob& J, int x, const ColK& g) {
+__device__ __forceinline__ float2 col_op(const AxisParams& A, const AxisJob& J, int x, const ColK& g, float lo) {
   const float kx = A.k[0][x];
   float kk = __fadd_rn(__fmul_rn(kx, kx), g.ky2);
   if (A.ndim == 3) kk = __fadd_rn(kk, g.kz2);
@@ -57,7 +57,7 @@ __device__ __forceinline__ float2 col_op(const AxisParams& A, const AxisJob& J, 
       v = A.us[J.axis][ai];
       break;
   }
-  return make_float2(v.x * A.scale, v.y * A.scale);
+  return make_float2(scaled(A, v.x, lo), scaled(A, v.y, lo));
 }
 
 // Strided axis: T = 256 / P columns per block, P threads per column.
@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(256) k_axis_reg(const __grid_constant__ AxisPa
     return;
   }
   const ColK g = col_geometry(A, act ? c0 + cc : c0);
+  const float lo = col_scale_lo(A, g.a1, g.a2, g.valid);
   int cur = -1;
   float2 X[E];
   for (int jj = 0; jj < A.njobs; ++jj) {
@@ -121,7 +122,7 @@ __global__ void __launch_bounds__(256) k_axis_reg(const __grid_constant__ AxisPa
 #pragma unroll
       for (int k2 = 0; k2 < P; ++k2) {
         float2 y = make_float2(0.f, 0.f);
-        if (act && g.valid) y = cconj(cmul(col_op(A, J, t + P * m + E * k2, g), X[m * P + k2]));
+        if (act && g.valid) y = cconj(cmul(col_op(A, J, t + P * m + E * k2, g, lo), X[m * P + k2]));
         Y[m * P + k2] = y;
       }
     kwreg::Reg<E, P>::rev(Y, t, sm, 1, tw, sync);

@@ -141,8 +141,9 @@ struct AxisParams {
   int use_kspace;
   float pow1, pow2;
   float scale;    // 1 / N_total
-  // mixed-radix passes: what the rounding of scale left out, and per axis and
-  // frequency -scale x the gain of the axis's transform pair (null: none)
+  // grids with mixed-radix passes: what the rounding of scale left out, less scale x the
+  // mean gain of axis 0 if that has power-of-two passes (other grids: 0), and per axis
+  // and frequency -scale x the gain of the axis's transform pair (null: none)
   float scale_lo;
   const float* eps[3];
   float nab_kk;   // a typical |k|^2 of the grid (scaling of logarithms)
@@ -176,6 +177,19 @@ __device__ __forceinline__ ColK col_geometry(const AxisParams& A, int c) {
   return g;
 }
 
+// The low part of 1 / (N_total gain) that is constant in a column: what the rounding
+// of scale left out and the gains of the other axes' transforms there.
+__device__ __forceinline__ float col_scale_lo(const AxisParams& A, int a1, int a2, bool valid) {
+  float lo = A.scale_lo;
+  if (!valid) return lo;
+  if (A.eps[1]) lo += __ldg(A.eps[1] + a1);
+  if (A.ndim == 3 && A.eps[2]) lo += __ldg(A.eps[2] + a2);
+  return lo;
+}
+
+// x / (N_total gain), rounded once; lo from col_scale_lo
+__device__ __forceinline__ float scaled(const AxisParams& A, float x, float lo) { return fmaf(x, A.scale, x * lo); }
+
 // Host launchers of the generic-length kernels (kw_generic.cuh: k_rows,
 // k_axis and their grouped forms, 256 threads per block), one set per FFT
 // schedule family F: 0 the Stockham stages (kw_kernels.cu), 1 the two-level
@@ -205,6 +219,8 @@ void kw_tma_plan_destroy(void* h);
 bool kw_tma_supported(int n);
 bool kw_tma_encode(void* h, int axis, int b, void* base, int ncols, int n, long long xs, int nouter, long long os, int P);
 cudaError_t kw_tma_attr(int n, int axis, bool small);
+// register-FFT shape of the plain passes of length n
+bool kw_tma_plain_shape(int n, int* E, int* P);
 // operator passes along `axis` on small tiles (set before encoding the maps)
 void kw_tma_set_small(void* h, int axis, bool small);
 bool kw_tma_small_wanted(int n, int ncols, int nsm);

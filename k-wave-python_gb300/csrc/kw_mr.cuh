@@ -233,6 +233,49 @@ inline void kw_mr_gain(const KwMrLen& L, const float2* w, double* eps) {
     }
 }
 
+// Gains of the two-level power-of-two passes (kw_regfft.cuh, n = E P), which share
+// grids with mixed-radix ones: E-point DFTs, the table twiddle w_n^{t k1}, P-point
+// DFTs; w: that table.  Entry (k, j) of their N-point DFT: N = N1 N2 with constant
+// twiddles rounded to float.
+inline void kw_reg_dft_entry(int N, int k, int j, double* re, double* im) {
+  if (N <= 4) {  // exact
+    const int q = (k * j) % N * (4 / N);
+    *re = q == 0 ? 1.0 : q == 2 ? -1.0 : 0.0;
+    *im = q == 1 ? -1.0 : q == 3 ? 1.0 : 0.0;
+    return;
+  }
+  const int N1 = N == 32 ? 8 : 4, N2 = N / N1, k1 = k % N1, k2 = k / N1, n1 = j / N2, n2 = j % N2;
+  double ar, ai, br, bi;
+  kw_reg_dft_entry(N1, k1, n1, &ar, &ai);
+  kw_reg_dft_entry(N2, k2, n2, &br, &bi);
+  const double c = (double)(float)kw_ct_trig(n2 * k1, N, false), s = -(double)(float)kw_ct_trig(n2 * k1, N, true);
+  const double tr = br * c - bi * s, ti = br * s + bi * c;
+  *re = tr * ar - ti * ai;
+  *im = tr * ai + ti * ar;
+}
+
+inline double kw_reg_dft_gain(int N, int k) {
+  double sum = 0.0;
+  for (int j = 0; j < N; ++j) {
+    double ar, ai, br, bi;
+    kw_reg_dft_entry(N, k, j, &ar, &ai);
+    kw_reg_dft_entry(N, j, k, &br, &bi);
+    sum += ar * br + ai * bi;
+  }
+  return sum / N - 1.0;
+}
+
+inline void kw_reg_gain(int E, int P, const float2* w, double* eps) {
+  for (int k1 = 0; k1 < E; ++k1) {
+    double g = kw_reg_dft_gain(E, k1);
+    for (int t = 0; t < P; ++t) {
+      const double c = w[t * k1].x, s = w[t * k1].y;
+      g += (c * c + s * s - 1.0) / P;
+    }
+    for (int k2 = 0; k2 < P; ++k2) eps[k1 + E * k2] = g + kw_reg_dft_gain(P, k2);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // register DFTs on packed two-lane adds (FADD2 / FFMA2)
 // ---------------------------------------------------------------------------

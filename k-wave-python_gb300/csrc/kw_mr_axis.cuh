@@ -170,18 +170,9 @@ __device__ __forceinline__ float mr_kappa(const AxisParams& A, float kk) {
   return kwreg::sinc_taylor_sq(y);
 }
 
-// x / (N_total gain) at x frequency kx, rounded once; lo from mr_col_lo
+// x / (N_total gain) at x frequency kx: scaled() with axis 0's own gain.
 __device__ __forceinline__ float mr_scaled(const AxisParams& A, float x, float lo, int kx) {
-  return fmaf(x, A.scale, x * (lo + __ldg(A.eps[0] + kx)));
-}
-
-// The low part of the scale that is constant in a column.
-__device__ __forceinline__ float mr_col_lo(const AxisParams& A, const ColK& g) {
-  float lo = A.scale_lo;
-  if (!g.valid) return lo;
-  if (A.eps[1]) lo += __ldg(A.eps[1] + g.a1);
-  if (A.ndim == 3 && A.eps[2]) lo += __ldg(A.eps[2] + g.a2);
-  return lo;
+  return scaled(A, x, lo + __ldg(A.eps[0] + kx));
 }
 
 // Column-constant 1-D factor of an operator along axis 1 or 2.
@@ -365,7 +356,7 @@ __device__ __forceinline__ void mr_axis_body(const MrAxisParams& W, int tile, in
     const float2* in = P.bufs[ib] + base;
     const ColK g = col_geometry(P, (int)c);
     const bool on = act && g.valid;
-    const float lo = mr_col_lo(P, g);
+    const float lo = col_scale_lo(P, g.a1, g.a2, g.valid);
     kwtma::grid_dep_wait();
     switch (L.r[0]) {
 #define KW_MR_CASE(R) \

@@ -106,6 +106,7 @@ struct kw_plan {
   float2* d_mr_tw_row = nullptr;
   uint32_t* d_mr_pos = nullptr;
   float* d_eps[3] = {nullptr, nullptr, nullptr};  // AxisParams::eps
+  double scale_rel = 0.0;  // relative correction of the scale for the mean gain of axis 0's register passes
   // persistent TMA axis passes
   void* tma = nullptr;
   bool tma_axis[3] = {false, false, false};
@@ -561,6 +562,28 @@ static void set_generic_geometry(kw_plan* p, int T_req, int R) {
   }
 }
 
+// Gain of a real row at its frequencies from that of its complex transform, c: its
+// frequency k goes through the complex frequencies k and M - k alike, and an even
+// row's odd part through its post twiddle.
+static std::vector<double> row_gain(const kw_plan* p, const std::vector<double>& c) {
+  const int M = p->Mfft;
+  std::vector<double> e(p->H);
+  for (int k = 0; k < p->H; ++k) {
+    e[k] = 0.5 * (c[k % M] + c[(M - k % M) % M]);
+    if (!p->even) continue;
+    const double a = -2.0 * M_PI * (double)k / (double)p->L, wr = (float)cos(a), wi = (float)sin(a);
+    e[k] += 0.5 * (wr * wr + wi * wi - 1.0);
+  }
+  return e;
+}
+
+// -scale x gain, as the operator passes read it
+static std::vector<float> gain_table(const kw_plan* p, const std::vector<double>& e) {
+  std::vector<float> f(e.size());
+  for (size_t k = 0; k < e.size(); ++k) f[k] = (float)(-e[k] / (double)p->ntot);
+  return f;
+}
+
 // Which lengths run on the mixed-radix passes (kw_mr.cuh): all that no
 // power-of-two kernel takes, and on 2-D grids and 3-D grids of up to 2^19
 // cells the power-of-two lengths too.  Those grids are bound by the latency of
@@ -586,9 +609,8 @@ static int setup_mr(kw_plan* p) {
   };
   size_t at_tw[3] = {0, 0, 0}, at_eps[3] = {0, 0, 0}, at_row = 0, at_pos = 0;
   bool any = false, has_eps[3] = {false, false, false};
-  auto push_eps = [&](int axis, const std::vector<double>& e) {  // -scale x eps, as the operator passes read it
-    std::vector<float> f(e.size());
-    for (size_t k = 0; k < e.size(); ++k) f[k] = (float)(-e[k] / (double)p->ntot);
+  auto push_eps = [&](int axis, const std::vector<double>& e) {
+    const std::vector<float> f = gain_table(p, e);
     at_eps[axis] = push(f.data(), f.size() * sizeof(float));
     has_eps[axis] = true;
   };
@@ -609,18 +631,9 @@ static int setup_mr(kw_plan* p) {
     const std::vector<uint32_t> pos = mr_positions(p->mr_row);
     at_row = push(w.data(), w.size() * sizeof(float2));
     at_pos = push(pos.data(), pos.size() * sizeof(uint32_t));
-    // a real row's frequency k goes through the complex frequencies k and M - k
-    // alike, and an even row's odd part through its post twiddle
-    const int M = p->Mfft;
-    std::vector<double> c(M), e(p->H);
+    std::vector<double> c(p->Mfft);
     kw_mr_gain(p->mr_row, w.data(), c.data());
-    for (int k = 0; k < p->H; ++k) {
-      e[k] = 0.5 * (c[k % M] + c[(M - k % M) % M]);
-      if (!p->even) continue;
-      const double a = -2.0 * M_PI * (double)k / (double)p->L, wr = (float)cos(a), wi = (float)sin(a);
-      e[k] += 0.5 * (wr * wr + wi * wi - 1.0);
-    }
-    push_eps(p->D - 1, e);
+    push_eps(p->D - 1, row_gain(p, c));
     p->rows_mr = true;
   }
   if (host.empty()) return KW_OK;
@@ -634,6 +647,31 @@ static int setup_mr(kw_plan* p) {
   if (p->rows_mr) {
     p->d_mr_tw_row = reinterpret_cast<float2*>(d + at_row);
     p->d_mr_pos = reinterpret_cast<uint32_t*>(d + at_pos);
+  }
+  return KW_OK;
+}
+
+// Gains of the power-of-two passes of a grid whose other axes run on mixed-radix
+// ones (grids of power-of-two passes alone keep their plain scale).  The y axis and
+// the rows get tables; of axis 0, whose operators would need one more table value
+// per point, the mean over its frequencies.
+static int setup_reg_gain(kw_plan* p) {
+  if (!p->d_eps[0] && !p->d_eps[1] && !p->d_eps[2]) return KW_OK;
+  for (int a = 0; a < p->D; ++a) {
+    const bool row = a == p->D - 1;
+    if (row ? p->rows_mr || !p->rows_reg : p->axis_mr[a] || (!p->tma_axis[a] && !p->axis_reg[a])) continue;
+    const int n = row ? p->Mfft : p->N[a];
+    int E = row ? p->rows_regE : p->axis_regE[a], P = row ? p->rows_regP : p->axis_regP[a];
+    if (!row && a == 1 && p->tma_axis[a]) kw_tma_plain_shape(n, &E, &P);
+    std::vector<double> e(n);
+    kw_reg_gain(E, P, twiddles(n, n).data(), e.data());
+    if (a == 0) {
+      for (double g : e) p->scale_rel -= g / n;
+      continue;
+    }
+    const std::vector<float> f = gain_table(p, row ? row_gain(p, e) : e);
+    int rc = upload(p, &p->d_eps[a], f.data(), f.size());
+    if (rc) return rc;
   }
   return KW_OK;
 }
@@ -856,6 +894,7 @@ int32_t kw_plan_finalize(kw_plan* p) {
       }
     }
   }
+  if ((rc = setup_reg_gain(p))) return rc;
   if ((rc = dalloc(p, &p->d_tstep, 1))) return rc;
   {
     const char* env = getenv("KWAVE_GB300_GRAPHS");
@@ -1180,8 +1219,10 @@ static int launch_axis_ops(kw_plan* p, const AxisJob* jobs, int nj, cudaStream_t
   A.pow2 = (float)(p->g.alpha_power - 1.0);
   const double scale = 1.0 / (double)p->ntot;
   A.scale = (float)scale;
-  A.scale_lo = (float)(scale - (double)A.scale);
-  for (int a = 0; a < 3; ++a) A.eps[a] = p->d_eps[a];
+  for (int a = 0; a < 3; ++a) {
+    A.eps[a] = p->d_eps[a];
+    if (A.eps[a]) A.scale_lo = (float)(scale - (double)A.scale + scale * p->scale_rel);
+  }
   {
     double kk = 0.0;
     for (int a = 0; a < p->D; ++a) kk += M_PI * M_PI / (3.0 * p->g.spacing[a] * p->g.spacing[a]);
