@@ -146,7 +146,11 @@ struct AxisParams {
   // and frequency -scale x the gain of the axis's transform pair (null: none)
   float scale_lo;
   const float* eps[3];
-  float nab_kk;   // a typical |k|^2 of the grid (scaling of logarithms)
+  // the same passes: tables and series of the fractional Laplacians (mr_kpow), their
+  // first eighth of an octave (the upper 12 bits of a float) and their length
+  const float4* kpow[2];
+  uint32_t kpow_first, kpow_n;
+  float kpow_b[2][6];
 };
 
 // Spectral operator for one column (ky, kz fixed) of the axis-0 pass.

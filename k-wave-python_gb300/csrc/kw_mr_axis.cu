@@ -1,8 +1,6 @@
 // Host side of the mixed-radix axis passes: pass kind, tile width, launch.
 #include "kw_mr_launch.cuh"
 
-#include <cmath>
-
 #define KW_MR_AXIS_DECL(name)                                                                                    \
   cudaError_t kw_mr_axis_attr_##name(int smem);                                                                  \
   cudaError_t kw_mr_axis_go_##name(dim3 grid, int threads, size_t smem, cudaStream_t st, const MrAxisParams* W,  \
@@ -74,15 +72,6 @@ cudaError_t kw_mr_axis_plan(const AxisParams& A, const KwMrLen& L, const float2*
     W.der = A.jobs[0].op;
     nitems = grad ? 1 : div ? D : nab ? A.njobs : ni;
     nbuf = (X.kind == MK_GRAD || X.kind == MK_GEN) ? 2 : 1;
-    if (X.kind == MK_NAB) {
-      // |k|^2 near 1 where most of the spectrum lies, so that its logarithm is
-      // small and keeps its low bits: a power of two near the mean |k|^2
-      const double kk = A.nab_kk > 0.f ? A.nab_kk : 1.0;
-      const int e = (int)std::lround(std::log2(kk));
-      W.nab_inv = (float)std::ldexp(1.0, -e);
-      W.nab_fac[0] = (float)std::exp2(0.5 * e * (double)A.pow1);
-      W.nab_fac[1] = (float)std::exp2(0.5 * e * (double)A.pow2);
-    }
   }
   W.lgT = mr_tile_log2(L, nbuf, W.ncoltot, nitems, nsm);
   const int T = 1 << W.lgT;

@@ -106,6 +106,9 @@ struct kw_plan {
   float2* d_mr_tw_row = nullptr;
   uint32_t* d_mr_pos = nullptr;
   float* d_eps[3] = {nullptr, nullptr, nullptr};  // AxisParams::eps
+  // |k|^p of the fractional Laplacians (AxisParams::kpow)
+  float4* d_kpow = nullptr;
+  uint32_t kpow_first = 0, kpow_n = 0;
   double scale_rel = 0.0;  // relative correction of the scale for the mean gain of axis 0's register passes
   // persistent TMA axis passes
   void* tma = nullptr;
@@ -651,6 +654,45 @@ static int setup_mr(kw_plan* p) {
   return KW_OK;
 }
 
+// Tables of |k|^p for the mixed-radix operator pass: every eighth of an octave that a
+// sum of squares of the wave numbers can lie in.
+static int setup_kpow(kw_plan* p) {
+  if (p->g.absorb_mode != 1 || !p->axis_mr[0]) return KW_OK;
+  auto eighth = [](float v) {
+    uint32_t b;
+    memcpy(&b, &v, 4);
+    return b >> 20;
+  };
+  float least = INFINITY, most = 0.f;
+  for (int a = 0; a < p->D; ++a) {
+    float top = 0.f;
+    for (float k : p->htab[KW_T_K][a]) {
+      const float k2 = k * k;
+      if (k2 > 0.f && std::isfinite(k2)) {
+        least = std::min(least, k2);
+        top = std::max(top, k2);
+      }
+    }
+    most += top;
+  }
+  if (!(least <= most)) least = most = 1.f;  // no wave number but 0
+  // (one more on either side for the rounding of the sums)
+  p->kpow_first = std::max(eighth(least), 1u) - 1;
+  p->kpow_n = std::min(eighth(most) + 1, 0x7f7u) - p->kpow_first + 1;
+  std::vector<float4> tab(2 * p->kpow_n);
+  for (int q = 0; q < 2; ++q)
+    for (uint32_t i = 0; i < p->kpow_n; ++i) {
+      const uint32_t lo = (p->kpow_first + i) << 20, hi = lo + (1u << 20) - 1;
+      float flo, fhi;
+      memcpy(&flo, &lo, 4);
+      memcpy(&fhi, &hi, 4);
+      const float rc = (float)(2.0 / ((double)flo + (double)fhi));
+      const double c = pow(1.0 / (double)rc, 0.5 * (p->g.alpha_power - (q == 0 ? 2.0 : 1.0)));
+      tab[q * p->kpow_n + i] = make_float4(rc, (float)c, (float)(c - (double)(float)c), 0.f);
+    }
+  return upload(p, &p->d_kpow, tab.data(), tab.size());
+}
+
 // Gains of the power-of-two passes of a grid whose other axes run on mixed-radix
 // ones (grids of power-of-two passes alone keep their plain scale).  The y axis and
 // the rows get tables; of axis 0, whose operators would need one more table value
@@ -839,6 +881,7 @@ int32_t kw_plan_finalize(kw_plan* p) {
     CK(cudaDeviceGetAttribute(&p->nsm, cudaDevAttrMultiProcessorCount, dev));
   }
   if ((rc = setup_mr(p))) return rc;
+  if ((rc = setup_kpow(p))) return rc;
   if (!p->generic_only) {
     const char* env = getenv("KWAVE_GB300_NO_TMA");
     const bool no_tma = env && env[0] == '1';
@@ -1223,10 +1266,15 @@ static int launch_axis_ops(kw_plan* p, const AxisJob* jobs, int nj, cudaStream_t
     A.eps[a] = p->d_eps[a];
     if (A.eps[a]) A.scale_lo = (float)(scale - (double)A.scale + scale * p->scale_rel);
   }
-  {
-    double kk = 0.0;
-    for (int a = 0; a < p->D; ++a) kk += M_PI * M_PI / (3.0 * p->g.spacing[a] * p->g.spacing[a]);
-    A.nab_kk = (float)kk;
+  if (p->d_kpow) {
+    A.kpow_first = p->kpow_first;
+    A.kpow_n = p->kpow_n;
+    for (int q = 0; q < 2; ++q) {
+      A.kpow[q] = p->d_kpow + (size_t)q * p->kpow_n;
+      const double hp = 0.5 * (p->g.alpha_power - (q == 0 ? 2.0 : 1.0));
+      double b = 1.0;  // binomial coefficients of (1 + z)^hp
+      for (int j = 0; j < 6; ++j) A.kpow_b[q][j] = (float)(b *= (hp - j) / (j + 1));
+    }
   }
   KwMrAxisLaunch X;
   if (p->axis_mr[0])
