@@ -275,6 +275,10 @@ int32_t kw_plan_read_series(kw_plan* plan, int32_t series, float* host, int64_t 
 int32_t kw_plan_read_aggregate(kw_plan* plan, int32_t series, int32_t kind, float* host, int64_t n);
 /* Whole field (p, u_i or rho_i), C order, N_total float32. */
 int32_t kw_plan_read_field(kw_plan* plan, int32_t field, float* host, int64_t n);
+/* The spectrum that the last step with a k-space corrected source in `slot`
+ * (KW_S_P0 or KW_S_U0..2) left, for tests: n = rows x padded half length x 2
+ * float32 (rows of N_last / 2 + 1 complex values, rounded up to even). */
+int32_t kw_plan_read_source_spectrum(kw_plan* plan, int32_t slot, float* host, int64_t n);
 /* Device pointer of a field (valid until kw_plan_destroy). */
 int32_t kw_plan_field_device_ptr(kw_plan* plan, int32_t field, void** dptr);
 /* Zeroes the state and the recorded series and rewinds to t = 0, keeping the

@@ -2082,11 +2082,16 @@ static int batch_graph(kw_batch* b, const std::vector<int>& keys, kw_batch::Grap
       int len = 0;
       for (int sl : {KW_S_P0, KW_S_U0, KW_S_U1, KW_S_U2})
         if (p->hsrc[sl].set && p->hsrc[sl].mode == KW_SRC_ADDITIVE) len = std::max(len, p->hsrc[sl].len);
-      for (auto& r : lists[i])
-        if (r.kind == 4 && r.ma.W.A.mode == 2 && r.ma.W.A.jobs[0].op == OP_SKAPPA) {
+      for (auto& r : lists[i]) {
+        if (r.kind != 4) continue;
+        const AxisParams& A = r.ma.W.A;
+        // (the y passes too: without the 1 / N of the kappa pass between them they
+        // multiply the spectrum that the last source step left by N_y a step)
+        if (A.mode == 2 ? A.jobs[0].op == OP_SKAPPA : A.plain[0] >= B_SRCP && A.plain[0] < B_US0) {
           r.ma.W.gate = p->d_tstep;
           r.ma.W.gate_end = len;
         }
+      }
       G.grouped[i] = 2;
       continue;
     }
@@ -2737,6 +2742,17 @@ int32_t kw_plan_read_field(kw_plan* p, int32_t field, float* host, int64_t n) {
   if (!d) return fail(KW_ERR_INVALID, "unknown field %d", field);
   if (n != p->ntot) return fail(KW_ERR_INVALID, "field buffer has %lld values, grid has %lld", (long long)n, p->ntot);
   CK(cudaMemcpy(host, d, n * sizeof(float), cudaMemcpyDeviceToHost));
+  return KW_OK;
+}
+
+int32_t kw_plan_read_source_spectrum(kw_plan* p, int32_t slot, float* host, int64_t n) {
+  if (!p || !host) return fail(KW_ERR_INVALID, "null argument");
+  if (!p->finalized) return fail(KW_ERR_STATE, "plan not finalized");
+  const int b = slot == KW_S_P0 ? (int)B_SRCP : slot >= KW_S_U0 && slot <= KW_S_U2 ? B_SRCU0 + slot - KW_S_U0 : -1;
+  if (b < 0 || !p->d_S[b]) return fail(KW_ERR_INVALID, "source slot %d has no spectrum", slot);
+  if (n != 2 * p->spec_elems)
+    return fail(KW_ERR_INVALID, "spectrum buffer has %lld values, expected %lld", (long long)n, 2 * p->spec_elems);
+  CK(cudaMemcpy(host, p->d_S[b], n * sizeof(float), cudaMemcpyDeviceToHost));
   return KW_OK;
 }
 

@@ -120,6 +120,7 @@ _PROTOS = {
     "kw_plan_read_series": (C.c_int32, [_P, C.c_int32, _P, C.c_int64]),
     "kw_plan_read_aggregate": (C.c_int32, [_P, C.c_int32, C.c_int32, _P, C.c_int64]),
     "kw_plan_read_field": (C.c_int32, [_P, C.c_int32, _P, C.c_int64]),
+    "kw_plan_read_source_spectrum": (C.c_int32, [_P, C.c_int32, _P, C.c_int64]),
     "kw_plan_field_device_ptr": (C.c_int32, [_P, C.c_int32, C.POINTER(_P)]),
     "kw_plan_reset": (C.c_int32, [_P]),
     "kw_plan_set_timing": (C.c_int32, [_P, C.c_int32]),
