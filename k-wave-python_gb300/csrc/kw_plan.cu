@@ -589,11 +589,16 @@ static std::vector<float> gain_table(const kw_plan* p, const std::vector<double>
 
 // Which lengths run on the mixed-radix passes (kw_mr.cuh): all that no
 // power-of-two kernel takes, and on 2-D grids and 3-D grids of up to 2^19
-// cells the power-of-two lengths too.  Those grids are bound by the latency of
-// each launch: 128^2 tissue 44 us a step against 60 on the TMA-fed kernels,
-// 512^2 70 against 85, 1024^2 120 against 169, 64^3 water 53 against 58; 128^3
-// tissue is the other way round (294 against 219).  KWAVE_GB300_MR=0: never,
-// =2: every length.
+// cells the power-of-two lengths too.  Small grids are bound by the latency of
+// each launch: us a step of tissue, these passes against the TMA-fed and
+// bulk-fed ones, 128^2 48 and 59, 512^2 71 and 84, 64^3 77 and 104, 64 x 64 x 128
+// (2^19 cells) 92 and 96, but 64 x 128 x 128 (2^20) 164 and 121, 128^3 284 and 208.
+// In 2-D it holds to the largest sizes: 1024 x 2048 261 and 328, 2048^2 453 and 846.
+// Rows of more than KW_MR_MAXM points are on the run-time-length kernel whatever the
+// columns take, and beside it power-of-two columns other than 512 stay where they
+// were: 256 x 2187 167 and 154, 64 x 2100 110 and 104, 1024 x 4096 1165 and 1137
+// (1024 x 3000 597 and 622); 512 x 2500 239 and 278, 512 x 4096 669 and 672.
+// KWAVE_GB300_MR=0: never, =2: every length.
 static int setup_mr(kw_plan* p) {
   if (p->generic_only) return KW_OK;
   const char* env = getenv("KWAVE_GB300_MR");
@@ -618,8 +623,11 @@ static int setup_mr(kw_plan* p) {
     has_eps[axis] = true;
   };
   int E, Pt;
+  const bool reg_rows = p->even && kw_reg_shape(p->Mfft, &E, &Pt);
+  const bool rows = (every || !reg_rows) && p->Mfft <= KW_MR_MAXM && kw_mr_factor(p->Mfft, p->mr_row, brief);
   for (int a = 0; a < p->D - 1; ++a) {
-    if ((!every && kw_reg_shape(p->N[a], &E, &Pt)) || !kw_mr_factor(p->N[a], p->mr_axis[a], brief)) continue;
+    const bool pow2_too = mode >= 2 || (every && (p->Mfft <= KW_MR_MAXM || p->N[a] == 512));
+    if ((!pow2_too && kw_reg_shape(p->N[a], &E, &Pt)) || !kw_mr_factor(p->N[a], p->mr_axis[a], brief)) continue;
     const std::vector<float2> w = mr_twiddles(p->mr_axis[a]);
     at_tw[a] = push(w.data(), w.size() * sizeof(float2));
     std::vector<double> e(p->N[a]);
@@ -628,8 +636,7 @@ static int setup_mr(kw_plan* p) {
     p->axis_mr[a] = any = true;
   }
   if (any && !kw_mr_axis_attr()) return fail(KW_ERR_CUDA, "mixed-radix kernel attributes: %s", cudaGetErrorString(cudaGetLastError()));
-  const bool reg_rows = p->even && kw_reg_shape(p->Mfft, &E, &Pt);
-  if ((every || !reg_rows) && p->Mfft <= KW_MR_MAXM && kw_mr_factor(p->Mfft, p->mr_row, brief)) {
+  if (rows) {
     const std::vector<float2> w = mr_twiddles(p->mr_row);
     const std::vector<uint32_t> pos = mr_positions(p->mr_row);
     at_row = push(w.data(), w.size() * sizeof(float2));
