@@ -1941,9 +1941,10 @@ static int batch_upload(kw_batch* b, const void* host, size_t bytes, void** out)
   return KW_OK;
 }
 
-// Plans whose passes all run on the mixed-radix kernels.
+// Plans whose passes all run on the mixed-radix kernels (in the wait test the
+// velocity stage does not).
 static bool mr_all(const kw_plan* p) {
-  if (!p->rows_mr) return false;
+  if (!p->rows_mr || p->wait_test) return false;
   for (int a = 0; a < p->D - 1; ++a)
     if (!p->axis_mr[a]) return false;
   return true;
