@@ -1518,6 +1518,7 @@ int32_t kw_unet_split_concat_grad(const void* dcat, int32_t nb, int32_t H, int32
 
 int32_t kw_unet_flip_weights(const void* w, void* wt, int32_t cout, int32_t cin, void* stream) {
   if (!w || !wt) return umma_fail(KW_ERR_INVALID, "kw_unet_flip_weights: null argument");
+  if (cout <= 0 || cin <= 0) return KW_OK;  // no weights
   k_flip_weights<<<dim3((cin + 31) / 32, (cout + 31) / 32, 9), dim3(32, 8), 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(wt), cout, cin);
   KW_UNET_CK();
