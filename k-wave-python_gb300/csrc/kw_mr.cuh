@@ -254,25 +254,37 @@ inline void kw_reg_dft_entry(int N, int k, int j, double* re, double* im) {
   *im = tr * ai + ti * ar;
 }
 
-inline double kw_reg_dft_gain(int N, int k) {
-  double sum = 0.0;
-  for (int j = 0; j < N; ++j) {
-    double ar, ai, br, bi;
-    kw_reg_dft_entry(N, k, j, &ar, &ai);
-    kw_reg_dft_entry(N, j, k, &br, &bi);
-    sum += ar * br + ai * bi;
-  }
-  return sum / N - 1.0;
+// Gains of the N-point DFT at its outputs (N a power of two up to 32, worked out once).
+inline const double* kw_reg_dft_gain(int N) {
+  struct Table {
+    double g[33][32];
+    Table() {
+      for (int n = 2; n <= 32; n *= 2)
+        for (int k = 0; k < n; ++k) {
+          double sum = 0.0;
+          for (int j = 0; j < n; ++j) {
+            double ar, ai, br, bi;
+            kw_reg_dft_entry(n, k, j, &ar, &ai);
+            kw_reg_dft_entry(n, j, k, &br, &bi);
+            sum += ar * br + ai * bi;
+          }
+          g[n][k] = sum / n - 1.0;
+        }
+    }
+  };
+  static const Table table;
+  return table.g[N];
 }
 
 inline void kw_reg_gain(int E, int P, const float2* w, double* eps) {
+  const double *ge = kw_reg_dft_gain(E), *gp = kw_reg_dft_gain(P);
   for (int k1 = 0; k1 < E; ++k1) {
-    double g = kw_reg_dft_gain(E, k1);
+    double g = ge[k1];
     for (int t = 0; t < P; ++t) {
       const double c = w[t * k1].x, s = w[t * k1].y;
       g += (c * c + s * s - 1.0) / P;
     }
-    for (int k2 = 0; k2 < P; ++k2) eps[k1 + E * k2] = g + kw_reg_dft_gain(P, k2);
+    for (int k2 = 0; k2 < P; ++k2) eps[k1 + E * k2] = g + gp[k2];
   }
 }
 
