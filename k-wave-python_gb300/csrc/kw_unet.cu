@@ -1039,8 +1039,10 @@ __global__ void __launch_bounds__(256) k_flip_weights(const __nv_bfloat16* __res
 
 // Bias gradient: db[c] += sum over pixels of dz[p][c].  Each block sums a range
 // of pixels, reduces per channel in shared memory and adds one value per channel
-// (red.add).  `vec` (C divides 2048, 16-byte aligned): a thread reads eight
-// channels at a time, always the same ones; otherwise one channel at a time.
+// (red.add).  `vec` (C a multiple of 8 up to 2048, 16-byte aligned): a thread reads
+// eight channels at a time, always the same ones; otherwise one channel at a time,
+// up to 256 channels always the same one (40 channels of 2^18 pixels 8.2 us, a thread
+// for a channel 126; 12 channels of 100,000 5.9 and 96).
 // Bound by DRAM at full resolution (67 MB: 17.4 -> 13.6 us) and by the number of
 // blocks at the deep layers (256 channels of 16 x 32^2, 16 blocks -> 512: 31 -> 3.7 us).
 __global__ void __launch_bounds__(256) k_bias_grad(const __nv_bfloat16* __restrict__ dz, float* __restrict__ db,
@@ -1049,7 +1051,8 @@ __global__ void __launch_bounds__(256) k_bias_grad(const __nv_bfloat16* __restri
   const long long p0 = (long long)blockIdx.x * pix_per_block;
   const long long p1 = min(npix, p0 + pix_per_block);
   if (vec) {
-    const int nv = C / 8;  // threads per pixel
+    const int nv = C / 8;            // threads per pixel
+    const int act = 256 / nv * nv;   // threads at work: whole pixels
     const long long v0 = p0 * nv, v1 = p1 * nv;
     const uint4* src = reinterpret_cast<const uint4*>(dz);
     float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -1061,27 +1064,66 @@ __global__ void __launch_bounds__(256) k_bias_grad(const __nv_bfloat16* __restri
         s[2 * j + 1] += __uint_as_float(w[j] & 0xffff0000u);
       }
     };
-    long long v = v0 + threadIdx.x;
-    for (; v + 768 < v1; v += 1024) {
-      const uint4 q0 = __ldg(src + v), q1 = __ldg(src + v + 256), q2 = __ldg(src + v + 512), q3 = __ldg(src + v + 768);
+    long long v = (int)threadIdx.x < act ? v0 + threadIdx.x : v1;
+    for (; v + 3 * act < v1; v += 4 * act) {
+      const uint4 q0 = __ldg(src + v), q1 = __ldg(src + v + act), q2 = __ldg(src + v + 2 * act),
+                  q3 = __ldg(src + v + 3 * act);
       take(q0);
       take(q1);
       take(q2);
       take(q3);
     }
-    for (; v < v1; v += 256) take(__ldg(src + v));
+    for (; v < v1; v += act) take(__ldg(src + v));
+    // sums of the same channels within a warp first, where nv divides 32 (8 channels: 9.4 -> 4.5 us)
+    const int lanes = nv < 32 && 32 % nv == 0 ? nv : 32;
+    for (int o = 16; o >= lanes; o >>= 1)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[threadIdx.x][j] = s[j];
     __syncthreads();
     for (int c = threadIdx.x; c < C; c += 256) {
       float t = 0.f;
-      for (int j = c >> 3; j < 256; j += nv) t += acc[j][c & 7];
+      for (int j = c >> 3; j < act; j += lanes < 32 ? 32 : nv) t += acc[j][c & 7];
       atomicAdd(db + c, t);
+    }
+  } else if (C <= 256) {
+    // thread t always meets channel t % C
+    const int act = 256 / C * C;
+    const long long e1 = p1 * C;
+    float s = 0.f;
+    if ((int)threadIdx.x < act) {
+      const __nv_bfloat16* z = dz + p0 * C;
+      const int ne = (int)(e1 - p0 * C);  // at most 1024 pixels of 256 channels
+      int e = threadIdx.x;
+      for (; e + 7 * act < ne; e += 8 * act) {
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = __bfloat162float(z[e + j * act]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s += v[j];
+      }
+      for (; e < ne; e += act) s += __bfloat162float(z[e]);
+    }
+    acc[threadIdx.x][0] = s;
+    __syncthreads();
+    if ((int)threadIdx.x < C) {
+      float t = 0.f;
+      for (int j = threadIdx.x; j < act; j += C) t += acc[j][0];
+      atomicAdd(db + threadIdx.x, t);
     }
   } else {
     for (int c = threadIdx.x; c < C; c += blockDim.x) {
       float t = 0.f;
-      for (long long p = p0; p < p1; ++p) t += __bfloat162float(dz[p * C + c]);
+      long long p = p0;
+      for (; p + 7 < p1; p += 8) {
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = __bfloat162float(dz[(p + j) * C + c]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) t += v[j];
+      }
+      for (; p < p1; ++p) t += __bfloat162float(dz[p * C + c]);
       atomicAdd(db + c, t);
     }
   }
@@ -1527,7 +1569,7 @@ int32_t kw_unet_flip_weights(const void* w, void* wt, int32_t cout, int32_t cin,
 
 int32_t kw_unet_bias_grad(const void* dz, float* db, int64_t npix, int32_t C, void* stream) {
   if (!dz || !db) return umma_fail(KW_ERR_INVALID, "kw_unet_bias_grad: null argument");
-  const int vec = C >= 8 && C <= 2048 && 2048 % C == 0 && aligned16(dz);
+  const int vec = C >= 8 && C <= 2048 && C % 8 == 0 && aligned16(dz);
   // pixels per block: about 600 blocks, at least four loads a thread and at most 1024 pixels one by one
   long long per = 1024;
   if (vec) per = std::max<long long>(8192 / C, (npix + 599) / 600);
