@@ -1547,7 +1547,10 @@ int32_t kw_unet_avgpool2_bwd(const void* dy, void* dx, int32_t nb, int32_t H, in
 int32_t kw_unet_relu_grad(const void* dy, const void* y, void* dz, int64_t n, void* stream) {
   if (!dy || !y || !dz) return umma_fail(KW_ERR_INVALID, "kw_unet_relu_grad: null argument");
   const long long nvec = aligned16(dy) && aligned16(y) && aligned16(dz) ? n / 8 : 0;
-  k_relu_grad<<<grid1(nvec ? (n + 31) / 32 : n), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  // a vector a thread for up to eight blocks an SM (a fifth of a million values: 3.0 us against
+  // 4.2 with four a thread), four a thread above
+  const long long work = nvec <= 8 * 152 * 256 ? nvec : (nvec + 3) / 4;
+  k_relu_grad<<<grid1(nvec ? work : n), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(y), static_cast<__nv_bfloat16*>(dz), n, nvec);
   KW_UNET_CK();
   return KW_OK;
