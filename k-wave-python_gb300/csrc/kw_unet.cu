@@ -444,7 +444,11 @@ __device__ __forceinline__ void fill_halo(const UmmaArgs& a, unsigned char* sA, 
 __host__ __device__ constexpr uint32_t acc_cols(int NT) { return NT <= 32 ? 32u : NT <= 64 ? 64u : NT <= 128 ? 128u : 256u; }
 __host__ __device__ constexpr uint32_t acc_count(int mode) { return mode == 5 ? 2u : 1u; }
 
-__global__ void __launch_bounds__(kThreads + 32, 2) k_umma(const __grid_constant__ UmmaArgs a, int* err) {
+// CTAS: resident CTAs per SM it is compiled for.  Two leave a gather thread the
+// registers to work ahead; three hide the fixed part of a tile where K is so
+// short that it dominates (umma_launch).
+template <int CTAS>
+__global__ void __launch_bounds__(kThreads + 32, CTAS) k_umma(const __grid_constant__ UmmaArgs a, int* err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   // stage s: A at base + s astage, B at base + S astage + s bstage
@@ -1211,22 +1215,23 @@ int g_umma_attr_dev = -1;
 int umma_fail(int code, const char* msg) { return kw_internal_fail(code, msg); }
 
 // Ring depth of a launch: as deep as two CTAs fit an SM's shared memory, or,
-// where that leaves fewer than three stages, one CTA.
+// where that leaves fewer than three stages, one CTA; no deeper than a CTA has
+// chunks, so that a third CTA fits where K is short (8 input channels: K = 72).
 int umma_stage_bytes(int NT, int mode) {
   return mode == 3 ? (int)kAHalo + NT * 288 : kATile + (mode >= 4 ? (NT + 63) / 64 * (int)kBlock : NT * kBK * 2);
 }
-int umma_stages(int NT, int mode) {
+int umma_stages(int NT, int mode, int chunks = kMaxStages) {
   const int b = umma_stage_bytes(NT, mode);
   const int two = 108 * 1024 / b, one = 220 * 1024 / b;
-  return std::min(kMaxStages, two >= 3 ? two : one);
+  return std::max(1, std::min({kMaxStages, two >= 3 ? two : one, chunks}));
 }
 
 // Dynamic shared memory of a launch: the stages, barriers and alignment slack
 // -- at least enough that no more CTAs share an SM than its 512 TMEM columns
 // hold (256-column tiles: 2 CTAs, 128-column tiles: 4), so that tcgen05.alloc
 // never has to wait.
-int umma_smem(int NT, int mode) {
-  const int need = umma_stages(NT, mode) * umma_stage_bytes(NT, mode) + 128 + 1024;
+int umma_smem(int NT, int mode, int chunks = kMaxStages) {
+  const int need = umma_stages(NT, mode, chunks) * umma_stage_bytes(NT, mode) + 128 + 1024;
   const int ncols = (int)(acc_cols(NT) * acc_count(mode));
   const int floor_bytes = ncols == 256 ? 80 * 1024 : ncols == 128 ? 48 * 1024 : 0;
   return need > floor_bytes ? need : floor_bytes;
@@ -1235,8 +1240,9 @@ int umma_smem(int NT, int mode) {
 int umma_launch(UmmaArgs& a, dim3 grid, cudaStream_t st) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return umma_fail(KW_ERR_CUDA, "cudaGetDevice failed");
-  const int smem = umma_smem(a.NT, a.mode);
-  a.stages = umma_stages(a.NT, a.mode);
+  const int chunks = a.mode == 3 ? (a.C1 + a.C2) / 16 : ((a.ksplit > 0 ? std::min(a.ksplit, a.K) : a.K) + kBK - 1) / kBK;
+  const int smem = umma_smem(a.NT, a.mode, chunks);
+  a.stages = umma_stages(a.NT, a.mode, chunks);
   if (a.H > 0) {
     a.dhw = kw_divu_make((uint32_t)(a.H * a.W));
     a.dw = kw_divu_make((uint32_t)a.W);
@@ -1245,11 +1251,17 @@ int umma_launch(UmmaArgs& a, dim3 grid, cudaStream_t st) {
     int most = 0;
     for (int nt = 16; nt <= kMaxNT; nt += 16)
       for (int mode : {0, 3, 4}) most = std::max(most, umma_smem(nt, mode));
-    if (cudaFuncSetAttribute(k_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
+    if (cudaFuncSetAttribute(k_umma<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess ||
+        cudaFuncSetAttribute(k_umma<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
       return umma_fail(KW_ERR_CUDA, "k_umma: cannot set the shared-memory size");
     g_umma_attr_dev = dev;
   }
-  k_umma<<<grid, kThreads + 32, smem, st>>>(a, kw_device_error_ptr());
+  // up to two chunks (convolutions of 8 channels, K = 72): 16 x 256^2 to 32 channels 158 us
+  // with two CTAs per SM, 123 with three; longer K is 10 % slower with three
+  if (chunks <= 2)
+    k_umma<3><<<grid, kThreads + 32, smem, st>>>(a, kw_device_error_ptr());
+  else
+    k_umma<2><<<grid, kThreads + 32, smem, st>>>(a, kw_device_error_ptr());
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     char buf[256];
