@@ -155,17 +155,18 @@ int32_t kw_plan_update_source(kw_plan* plan, int32_t slot, const float* signal, 
 int32_t kw_plan_finalize(kw_plan* plan);
 /* Advances min(nsteps, Nt - t) steps of Simulation.step (kspace_solver.py:691-747)
  * on `stream` (a cudaStream_t, NULL = default stream); returns after enqueueing.
- * Steps with the same launch sequence run as one CUDA graph, captured on first
- * use and replayed with the step index held on the device; the last step of a
+ * Steps with the same launch sequence run as CUDA graphs of one step, or of
+ * eight in runs of 32 and more, captured on first use and replayed with the
+ * step index held on the device; the last step of a
  * call, the t = 0 initial-condition step and every step while timing is on are
  * plain launches.  Use one stream per plan. */
 int32_t kw_plan_run(kw_plan* plan, int32_t nsteps, void* stream);
-/* Autotuner of the run-time-length FFT kernels (lengths with a prime factor
- * above 7, and plans of KW_DESC_GENERIC_FFT): times `nsteps` graph steps after the t = 0 step (at least
- * 2, at most Nt - 1) for each candidate launch geometry -- tile columns T in
- * {2, 4, 8, 16} of the axis passes, rows per block R in {R0/2, R0, 2 R0} of
- * the row stages -- keeps the fastest and rewinds the plan to t = 0
- * (kw_plan_reset).  The plan must be at
+/* Autotuner of the run-time-length FFT kernels (rows of more than 1024 complex
+ * points, axes of 2, 3, 5 or 7 points, and plans of KW_DESC_GENERIC_FFT): times
+ * `nsteps` graph steps after the t = 0 step (at least 2, at most Nt - 1) for
+ * each candidate launch geometry -- tile columns T in {2, 4, 8, 16} of the axis
+ * passes, rows per block R in {R0/2, R0, 2 R0} of the row stages -- keeps the
+ * fastest and rewinds the plan to t = 0 (kw_plan_reset).  The plan must be at
  * t = 0.  Results are bit-identical for every choice.  *T_out / *R_out (may be
  * NULL) receive the geometry in use; plans without such kernels are left as
  * they are. */
@@ -217,9 +218,10 @@ int32_t kw_plan_set_graphs(kw_plan* plan, int32_t enable);
  * no counterpart in the reference, which runs one Simulation at a time).
  * kw_batch_run advances every plan by min(nsteps, Nt - t) steps; each step of
  * all plans whose steps are graph steps is ONE graph launch.  Inside it the
- * passes of plans created with KW_DESC_GENERIC_FFT are grouped: the k-th
- * launch of every such plan's step runs in one grouped launch; other plans
- * join as parallel branches holding their own step graphs.  Plans keep their
+ * plans whose passes all run on the mixed-radix kernels share grouped launches
+ * (the k-th launch of every such plan's step) in up to three chains beside each
+ * other, and those created with KW_DESC_GENERIC_FFT in one; other plans join
+ * as parallel branches holding their own step graphs.  Plans keep their
  * own state, results and read functions.  Destroy the batch before its plans. */
 typedef struct kw_batch kw_batch;
 int32_t kw_batch_create(kw_plan* const* plans, int32_t n, kw_batch** out);

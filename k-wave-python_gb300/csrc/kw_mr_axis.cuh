@@ -171,7 +171,7 @@ __device__ __forceinline__ float mr_kappa(const AxisParams& A, float kk) {
 // |k|^p from |k|^2 (0 at k = 0), p the exponent of fractional Laplacian q: with the
 // centre c of the eighth of an octave that |k|^2 lies in, c^(p/2) (1 + z)^(p/2), z =
 // |k|^2 / c - 1, |z| <= 1/17.  c^(p/2) comes from a table in two parts, the rest is the
-// binomial series to z^6 (its next term is below 1e-10), so that nothing but the last
+// binomial series to z^6 (its next term is below 2e-9), so that nothing but the last
 // addition rounds to float: errors of 2.5e-8 rms and 6.2e-8 at most for p -1.4 to 0.9,
 // against 2.0e-8..4.5e-8 and 1.5e-7 for powf(|k|, p) behind a square root and
 // 4.1e-8..7.9e-8 and 6e-7, with a mean of up to 6e-8, for exp2f(p/2 log2f(|k|^2)).

@@ -29,7 +29,8 @@
 #define KW_MR_THREADS 192  // most threads of a row block
 #define KW_MR_MAXM 1024    // most points of a sequence
 // Most dynamic shared memory of a row block: one sequence of 1024 points in each
-// of up to six regions, slots of up to 16 / 15 of the points.
+// of up to six regions, slots of up to 3 / 2 of the points (a last radix of 2 is
+// padded to 3): 72 KB.
 #define KW_MR_ROWS_SMEM (96 * 1024)
 
 struct MrRowsParams {

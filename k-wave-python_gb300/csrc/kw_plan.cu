@@ -1722,7 +1722,7 @@ static void adj_swap(kw_plan* p, float*& lp, float** lu, float** lr, float*& res
 
 // The gradient of <residual, recorded p> for the lossless, source-free loop:
 // the transposed steps t = Nt-1 .. 1 and the transposed t = 0 override
-// (adjoint_body in kw_kernels.cu) on the run-time-length row kernels, with the
+// (adjoint_body in kw_generic.cuh) on the plan's own row and axis kernels, with the
 // adjoint state in buffers of its own.  With grad_c, the forward density sum
 // of every step is regenerated from the checkpoints, segment by segment from
 // the last (restore slot s, rerun its steps, keep sum_i rho_i of each), and

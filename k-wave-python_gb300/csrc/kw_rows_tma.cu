@@ -35,9 +35,8 @@
 namespace {
 
 constexpr uint64_t kRowWaitNs = 2000000000ull;
-// Ring depth and resident CTAs per SM per stage: the density stage keeps its
-// density-sum slots in shared memory and needs more registers (2 CTAs, 4
-// slots); the velocity and EOS stages run 3 CTAs of 3 slots.
+// Ring depth and resident CTAs per SM per stage: three CTAs of three slots, of
+// two for the density stages, which keep their density sums in shared memory.
 __host__ __device__ constexpr int row_nst(int stage) { return stage == ST_RHO_PL || stage == ST_RHO ? 2 : 3; }
 __host__ __device__ constexpr int row_ctas(int stage) { return 3; }
 

@@ -381,8 +381,10 @@ class SimulationBatch:
 
     Each member keeps its own grid size, medium, sources, sensor and results.
     Every step of all members is one CUDA graph launch.  By default each
-    member uses the kernels picked for its grid and joins that graph as a
-    parallel branch holding its own step graph.  With ``grouped=True`` the
+    member uses the kernels picked for its grid; members whose passes all run
+    on the mixed-radix kernels share grouped launches, in up to three chains,
+    and the others join the graph as parallel branches holding their own step
+    graphs.  With ``grouped=True`` the
     members set up here use the run-time-length FFT kernels, and the k-th pass
     of every member runs in one grouped launch over all of them (a handful of
     launches per step whatever the batch size).  ``autotune=True`` times
