@@ -2,7 +2,6 @@
 #include "kw_mr_launch.cuh"
 
 #define KW_MR_AXIS_DECL(name)                                                                                    \
-  cudaError_t kw_mr_axis_attr_##name(int smem);                                                                  \
   cudaError_t kw_mr_axis_go_##name(dim3 grid, int threads, size_t smem, cudaStream_t st, const MrAxisParams* W,  \
                                    const MrAxisParams* Ps, const int2* map, bool pdl);
 KW_MR_AXIS_DECL(fwd)
@@ -13,8 +12,6 @@ KW_MR_AXIS_DECL(nab)
 KW_MR_AXIS_DECL(gen)
 
 namespace {
-constexpr int kMrSmemMax = 160 * 1024;
-
 // Columns per block (a power of two) for `nbuf` column buffers of length L:
 // 16 (a row of a tile is then one 128-byte line) as long as three blocks of
 // plain passes fit an SM, fewer for long axes; halved down to 4 (one 32-byte
@@ -26,12 +23,6 @@ int mr_tile_log2(const KwMrLen& L, int nbuf, long long ncoltot, int nitems, int 
   return lg;
 }
 }  // namespace
-
-bool kw_mr_axis_attr() {
-  return kw_mr_axis_attr_fwd(kMrSmemMax) == cudaSuccess && kw_mr_axis_attr_inv(kMrSmemMax) == cudaSuccess &&
-         kw_mr_axis_attr_grad(kMrSmemMax) == cudaSuccess && kw_mr_axis_attr_div(kMrSmemMax) == cudaSuccess &&
-         kw_mr_axis_attr_nab(kMrSmemMax) == cudaSuccess && kw_mr_axis_attr_gen(kMrSmemMax) == cudaSuccess;
-}
 
 // Parameters and launch shape of one pass along an axis: A in plain mode over
 // `nb` buffers, or its job list; nouter outer blocks of A.ncols columns; nsm
@@ -80,7 +71,7 @@ cudaError_t kw_mr_axis_plan(const AxisParams& A, const KwMrLen& L, const float2*
   X.threads = (per * T + 31) / 32 * 32;
   if (X.threads > 256) X.threads = 256;
   X.smem = ((size_t)L.slots * sizeof(float2) << W.lgT) * nbuf;
-  if (X.smem > (size_t)kMrSmemMax) return cudaErrorInvalidValue;
+  if (X.smem > KW_MR_AXIS_SMEM) return cudaErrorInvalidValue;
   W.gx = X.gx = (int)((W.ncoltot + T - 1) / T);
   X.gy = nitems;
   return cudaSuccess;

@@ -22,6 +22,8 @@
 #include "kw_regfft.cuh"
 #include "kw_tma.cuh"
 
+#define KW_MR_AXIS_SMEM (160 * 1024)  // most dynamic shared memory of a block
+
 enum KwMrKind { MK_FWD = 0, MK_INV = 1, MK_GRAD = 2, MK_DIV = 3, MK_NAB = 4, MK_GEN = 5 };
 
 struct MrAxisParams {
@@ -487,23 +489,24 @@ __global__ void __launch_bounds__(256, (KIND == MK_GRAD || KIND == MK_GEN) ? 2 :
   mr_axis_body<KIND>(sp, me.y - item * sp.gx, item);
 }
 
-template <int KIND>
-static cudaError_t kw_mr_axis_attr_kind(int smem) {
-  cudaError_t e = cudaFuncSetAttribute(k_mr_axis<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_mr_axis_group<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  return e;
-}
-
-// One plan's pass, or (Ps set) the grouped pass over `grid.x` blocks.
+// One plan's pass, or (Ps set) the grouped pass over `grid.x` blocks.  Only a launch
+// that needs it asks for more shared memory (one constant, so that plans of several
+// threads never lower it): the call loads the kernel, and a first 2-D run that asked
+// for all twelve at set-up took 10 ms longer.
 template <int KIND>
 static cudaError_t kw_mr_axis_go(dim3 grid, int threads, size_t smem, cudaStream_t st, const MrAxisParams* W,
                                  const MrAxisParams* Ps, const int2* map, bool pdl) {
+  if (smem > 40 * 1024) {
+    const cudaError_t e =
+        Ps ? cudaFuncSetAttribute(k_mr_axis_group<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, KW_MR_AXIS_SMEM)
+           : cudaFuncSetAttribute(k_mr_axis<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, KW_MR_AXIS_SMEM);
+    if (e != cudaSuccess) return e;
+  }
   if (Ps) return kwtma::launch_k(k_mr_axis_group<KIND>, grid, dim3(threads), smem, st, pdl, Ps, map);
   return kwtma::launch_k(k_mr_axis<KIND>, grid, dim3(threads), smem, st, W->pdl != 0, *W);
 }
 
 #define KW_MR_AXIS_DEFINE(name, KIND)                                                                              \
-  cudaError_t kw_mr_axis_attr_##name(int smem) { return kw_mr_axis_attr_kind<KIND>(smem); }                        \
   cudaError_t kw_mr_axis_go_##name(dim3 grid, int threads, size_t smem, cudaStream_t st, const MrAxisParams* W,    \
                                    const MrAxisParams* Ps, const int2* map, bool pdl) {                            \
     return kw_mr_axis_go<KIND>(grid, threads, smem, st, W, Ps, map, pdl);                                          \

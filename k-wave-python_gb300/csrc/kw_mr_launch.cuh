@@ -16,7 +16,6 @@ struct KwMrRowsLaunch {
   size_t smem;
 };
 
-bool kw_mr_axis_attr();
 // cudaErrorInvalidValue when a job of A writes another job's input
 cudaError_t kw_mr_axis_plan(const AxisParams& A, const KwMrLen& L, const float2* tw, int nouter, int nb, int nsm,
                             KwMrAxisLaunch& X);

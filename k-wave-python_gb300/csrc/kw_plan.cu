@@ -616,7 +616,7 @@ static int setup_mr(kw_plan* p) {
     return at;
   };
   size_t at_tw[3] = {0, 0, 0}, at_eps[3] = {0, 0, 0}, at_row = 0, at_pos = 0;
-  bool any = false, has_eps[3] = {false, false, false};
+  bool has_eps[3] = {false, false, false};
   auto push_eps = [&](int axis, const std::vector<double>& e) {
     const std::vector<float> f = gain_table(p, e);
     at_eps[axis] = push(f.data(), f.size() * sizeof(float));
@@ -633,9 +633,8 @@ static int setup_mr(kw_plan* p) {
     std::vector<double> e(p->N[a]);
     kw_mr_gain(p->mr_axis[a], w.data(), e.data());
     push_eps(a, e);
-    p->axis_mr[a] = any = true;
+    p->axis_mr[a] = true;
   }
-  if (any && !kw_mr_axis_attr()) return fail(KW_ERR_CUDA, "mixed-radix kernel attributes: %s", cudaGetErrorString(cudaGetLastError()));
   if (rows) {
     const std::vector<float2> w = mr_twiddles(p->mr_row);
     const std::vector<uint32_t> pos = mr_positions(p->mr_row);
@@ -924,7 +923,7 @@ int32_t kw_plan_finalize(kw_plan* p) {
     }
     for (int a = 0; a < D - 1; ++a) {
       p->axis_reg[a] = kw_reg_shape(p->N[a], &p->axis_regE[a], &p->axis_regP[a]);
-      if (p->axis_reg[a]) CK(kw_axis_reg_attr(p->N[a]));
+      if (p->axis_reg[a] && !p->axis_mr[a]) CK(kw_axis_reg_attr(p->N[a]));
     }
     if (p->even) {
       // the register row kernels index pairs with 32 bits
@@ -935,10 +934,11 @@ int32_t kw_plan_finalize(kw_plan* p) {
         int rs = p->Mfft + p->rows_regE;
         while (rs % 16 != target) ++rs;
         p->rows_RS = rs;
-        CK(kw_rows_v2_attr(p->Mfft));
+        // (kernels that the plan does not use are not loaded for it)
+        if (!p->rows_mr) CK(kw_rows_v2_attr(p->Mfft));
         const char* env = getenv("KWAVE_GB300_ROWS_TMA");
         if (!(env && env[0] == '0') && kw_device_error_ptr()) {
-          CK(kw_rows_tma_attr(p->Mfft, p->Hp, p->rows_RS));
+          if (!p->rows_mr) CK(kw_rows_tma_attr(p->Mfft, p->Hp, p->rows_RS));
           p->rows_tma = true;
         }
       }
@@ -1862,6 +1862,7 @@ int32_t kw_plan_set_wait_test(kw_plan* p, int32_t enable) {
   if (enable && !p->rows_tma)
     return fail(KW_ERR_UNSUPPORTED, "the wait test needs the bulk-fed row stages (a power-of-two last axis)");
   CK(cudaDeviceSynchronize());
+  if (enable && p->rows_mr) CK(kw_rows_tma_attr(p->Mfft, p->Hp, p->rows_RS));
   p->wait_test = enable != 0;
   drop_graphs(p);  // captured steps hold the launch parameters
   return KW_OK;
