@@ -22,7 +22,9 @@ SOURCES = ["kw_kernels.cu", "kw_generic_fft2.cu", "kw_axis_tma.cu", "kw_axis_tma
            "kw_mr_rows.cu", "kw_mr_rows1.cu", "kw_mr_rows2.cu", "kw_mr_rows3.cu", "kw_mr_rows4.cu", "kw_mr_rows5.cu",
            "kw_rows_reg.cu", "kw_rows_reg2.cu", "kw_rows_reg3.cu", "kw_rows_tma.cu", "kw_plan.cu", "kw_noalloc.cu", "kw_unet.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "--extended-lambda"]
+# (device code is stored as it is: unpacking its line tables when a kernel is first used
+# took longer than running it -- first 375 x 324 transmit of a process 46 ms, so 23)
+NVCC_FLAGS = ["-O3", "-lineinfo", "--compress-mode=none", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "--extended-lambda"]
 
 
 def _nvcc():
